@@ -43,6 +43,20 @@ as_status scratch(as_ctx *ctx, size_t bytes, void **out) {
     return AS_OK;
 }
 
+as_status scratch_list(as_ctx *ctx, long n, cudaStream_t s, int **out) {
+    const size_t bytes = static_cast<size_t>(n) * sizeof(int);
+    *out = nullptr;
+    if (bytes > ctx->scratch_bytes) {
+        cudaStreamCaptureStatus cap = cudaStreamCaptureStatusNone;
+        if (cudaStreamIsCapturing(s, &cap) != cudaSuccess || cap != cudaStreamCaptureStatusNone)
+            return AS_OK;
+    }
+    void *p = nullptr;
+    const as_status st = scratch(ctx, bytes, &p);
+    if (st == AS_OK) *out = static_cast<int *>(p);
+    return st;
+}
+
 struct DeviceGuard {
     int prev = -1;
     explicit DeviceGuard(int dev) {

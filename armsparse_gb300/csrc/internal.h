@@ -37,6 +37,10 @@ as_status check_cuda(cudaError_t e, const char *what);
 // pointer that earlier work still holds.
 as_status scratch(as_ctx *ctx, size_t bytes, void **out);
 
+// A scratch list of n ints, or nullptr (and AS_OK) when the arena would have to grow while the
+// stream is being captured: the caller then runs without a list.
+as_status scratch_list(as_ctx *ctx, long n, cudaStream_t s, int **out);
+
 // ---- launchers (return AS_OK or an error; count launches in ctx) ----
 struct SpmmArgs {
     int M, K, N, nnz;
@@ -82,16 +86,13 @@ as_status spmm_nnzme_launch(as_ctx *ctx, int dtype, int vb, int group, int chunk
                             const SpmmArgs &a, cudaStream_t s, const SddmmFuse *fuse = nullptr);
 as_status spmm_bulk_launch(as_ctx *ctx, int dtype, int lane_bytes, int stages, const SpmmArgs &a,
                            cudaStream_t s);
-// Long rows of the row-split kernels: the cp.async size (16 or 4 bytes) the layout allows,
-// 0 when none does; the launch of the kernel that takes the listed rows.
-int spmm_long_granule(int dtype, int N, long ldb, const void *B);
+// The kernel that takes the long rows that a row-oriented kernel listed (any layout).
 // `op` is the chain's step: 0 the SpMM's fused multiply-add, 1 the unweighted sum, 2 max from
 // -inf, 3 the DGL max (spmm_reduce.cu's reductions), 4 the fused multiply-add skipping zero
 // values (spmm_vcsr4.cu's empty slots), 5 the row-pair layout's two chains per listed pair
 // (spmm_rowpair.cu; `pair_flag` is its flag array); the steps other than 0 take fp32.
-as_status spmm_long_launch(as_ctx *ctx, int dtype, int granule, const SpmmArgs &a,
-                           const int *list, cudaStream_t s, int op = 0,
-                           const uint8_t *pair_flag = nullptr);
+as_status spmm_long_launch(as_ctx *ctx, int dtype, const SpmmArgs &a, const int *list,
+                           cudaStream_t s, int op = 0, const uint8_t *pair_flag = nullptr);
 as_status spgemm_dense_launch(as_ctx *ctx, int M, int K, int N, int nnz_a, const int *rp1,
                               const int *ci1, const float *v1, int nnz_b, const int *rp2,
                               const int *ci2, const float *v2, float *C, long ldc, float beta,

@@ -9,9 +9,8 @@
 //   in CSR order and updates its accumulators with fmaf(b, v, acc). Each output element is
 //   therefore exactly the reference's fused-FMA chain. Blocks are 256 threads; blockIdx.x
 //   runs over row blocks and blockIdx.y over column tiles, so the CTAs resident at any
-//   moment share one column tile of B, which stays in L2. Rows with more than kLongRow
-//   entries are skipped here and computed by the long-row kernel (spmm_long.cu), which keeps
-//   the same chains.
+//   moment share one column tile of B, which stays in L2. Long rows (long_row_threshold) are
+//   skipped here and computed by the long-row kernel (spmm_long.cu), which keeps the same chains.
 #include <limits.h>
 #include <stdio.h>
 
@@ -458,16 +457,13 @@ as_status spmm_launch(as_ctx *ctx, int dtype, int variant, const SpmmArgs &a, cu
                                             " needs N, ldb, ldc and pointer alignment to match its vector width");
     if (ceil_div(a.N, (v.vb / (dtype == 0 ? 4 : 2)) * v.group * v.cpl) > 65535)
         return fail(AS_ERR_UNSUPPORTED, "spmm: N too large for this variant's column tile");
-    // rows longer than kLongRow entries go to the long-row kernel when its copies can serve
-    // the layout (a matrix with nnz <= kLongRow has none)
+    // long rows go to the long-row kernel (a matrix of fewer entries than one has none)
     LongRows lr{INT_MAX, nullptr, ctx->d_long};
-    const int granule = a.nnz > kLongRow && a.M > 0 ? spmm_long_granule(dtype, a.N, a.ldb, a.B) : 0;
-    if (granule) {
-        void *p = nullptr;
-        as_status st = scratch(ctx, static_cast<size_t>(a.M) * sizeof(int), &p);
+    const int thresh = long_row_threshold(a.nnz, a.M);
+    if (a.nnz > thresh && a.M > 0) {
+        as_status st = scratch_list(ctx, a.M, s, &lr.list);
         if (st != AS_OK) return st;
-        lr.thresh = kLongRow;
-        lr.list = static_cast<int *>(p);
+        if (lr.list) lr.thresh = thresh;
     }
     bool ok = false;
     if (v.pf) {
@@ -490,8 +486,8 @@ as_status spmm_launch(as_ctx *ctx, int dtype, int variant, const SpmmArgs &a, cu
     if (!ok) return fail(AS_ERR_UNSUPPORTED, "spmm: variant not instantiated");
     ctx->launches++;
     as_status st = check_cuda(cudaGetLastError(), "spmm launch");
-    if (st != AS_OK || !granule) return st;
-    st = spmm_long_launch(ctx, dtype, granule, a, lr.list, s);
+    if (st != AS_OK || !lr.list) return st;
+    st = spmm_long_launch(ctx, dtype, a, lr.list, s);
     if (st != AS_OK) cudaMemsetAsync(ctx->d_long, 0, 3 * sizeof(unsigned), s);
     return st;
 }

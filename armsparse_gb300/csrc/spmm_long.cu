@@ -11,164 +11,221 @@
 // The same kernel takes the long rows of the other row-oriented SpMMs, with their own chain
 // step (OP below): the reduce aggregations (spmm_reduce.cu), the 1x4-blocked layout
 // (spmm_vcsr4.cu) and the row-pair layout (spmm_rowpair.cu: a listed pair gives a unit per
-// row, whose chain runs over the entries a per-stage include mask keeps).
+// row, whose chain runs over the entries that the unit includes).
 //
 // Each output element is still one chain over the row's entries in CSR order (the order
-// cannot be split without changing the bits), so the speed comes from feeding the chains. A
-// CTA takes one (long row, 64-column slice) at a time; its warps split by role:
-//  - warp 0 is the consumer: lane l runs the chains of columns 2l and 2l+1 of the slice out of
-//    shared memory, stage after stage (kStage entries per stage), reading each entry's two B
-//    values with one 64-bit (fp32) or 32-bit (bf16) load and the entry's value from the
-//    stage's value slot. It waits for a stage on the slot's `full` flag (an acquire load of a
-//    shared word) and frees the slot by a release store to its `empty` flag;
-//  - eight producer warps take the stages in turn (warp p owns stages p, p + 8, ..., all in
-//    slot p). For its stage a warp waits for the slot's `empty` flag, stores the entries'
-//    values (loaded into registers one turn earlier) into the value slot, and copies each
-//    entry's B segment into the ring slot with cp.async, eight lanes per entry; the entries'
-//    column indices, also loaded one turn earlier, reach those lanes by shuffle. It then waits
-//    for its own copies (cp.async.wait_group 0; its next stage is a whole turn away) and
-//    lane 0 publishes the stage with a release store to the slot's `full` flag after
-//    __syncwarp.
-// The consumer warp sits alone on its SM sub-partition (warps 4 and 8 are idle): the chains
-// issue one FMA every few cycles and lose a large share of that rate when two busy producer
-// warps share its scheduler.
+// cannot be split without changing the bits): the floor of a row is its length times the
+// latency of one fused multiply-add (4 cycles), and the kernel's work is to keep that chain
+// fed. A unit is a (long row, column slice); a slice is 32 words of a row of B (32 fp32 or 64
+// bf16 columns). A CTA walks its units as one stream of blocks of kBlk entries, without a
+// barrier between units; its warps split by role:
+//  - warp 0 is the consumer: lane l runs the chains of its one (fp32) or two (bf16) columns out
+//    of shared memory. A slot holds the block transposed by fours: the words of four
+//    consecutive entries of one lane lie together, so one 16-byte read brings four entries and
+//    the chain is not held up by the rate at which one warp issues shared-memory reads (32-bit
+//    reads: 5.8 cycles per entry; 128-bit reads: 4.5). The 16 entries after the ones whose
+//    steps run are always being read meanwhile, also across the end of a block, and the next
+//    block's barrier is tested a block ahead;
+//  - six producer warps take the blocks in turn. For its block a warp loads the entries'
+//    segments (all kBlk in flight; the indices were loaded one turn earlier), 16 bytes per lane
+//    and four entries per load where the layout allows, waits until the slot's last block has
+//    been consumed, and stores segments and values (word c of a segment belongs to consumer
+//    lane c % 4 * 8 + c / 4, which makes these stores free of bank conflicts). Positions that add nothing (past a row's end, or entries a row-pair unit leaves
+//    out) get the word -0.0 and the value 1, which keep every accumulator as it is, so the
+//    consumer runs one form of the step.
+// The consumer shares its SM sub-partition with an idle warp only (warp 4): the chain issues
+// one step every four cycles and loses a share of that rate to every busy neighbour.
 //
-// Every wait is bounded; a wait that gives up sets the timeout flag and an abort flag that makes
-// the other role leave too. No copy is ever in flight when a warp leaves (a stage is published
-// only after its copies landed); a row whose wait gave up is left unwritten. A malformed column
-// index is flagged and its entry gets a zero segment (nothing is read for it).
+// Measured on GB300: one row of 300,000 entries takes 1.02 ms over 32 fp32 columns (6.8 cycles per
+// entry at 2070 MHz; 64-column slices read 32 bits at a time, copied by cp.async and handed over
+// through flags: 1.9 ms, 13 cycles), 1.27 ms where B (153 MB) comes from DRAM, 1.67 ms where B's
+// rows allow 4-byte loads only. The loads of a block are volatile because their order is the
+// point: left to the compiler, they were moved down to their uses (3.1 ms in place of 1.3), as
+// was each load put under a condition of its own (5.1 ms in place of 1.7).
+//
+// Every wait is bounded; a wait that gives up sets the timeout flag and an abort flag that
+// makes the other role leave too; a row whose wait gave up is left unwritten. Loads land in
+// registers, so nothing is in flight when a warp leaves. A malformed column index is flagged
+// and its entry gets a zero segment (nothing is read for it).
 //
 // The list counters and a CTA-done counter live in the context's device words; the last CTA
 // to finish resets them, so the next call starts from zero without a memset.
 #include <algorithm>
+#include <math.h>
 
 #include "common.cuh"
 #include "internal.h"
+#include "spmm_vec.cuh"
 
 namespace as {
 namespace {
 
-constexpr int kCols = 64;                   // columns per slice (two per consumer lane)
-constexpr int kStage = 64;                  // entries per pipeline stage
-constexpr int kStages = 8;                  // ring slots
-constexpr int kProducers = 8;               // producer warps, one stage each in turn
-constexpr int kWarps = 12;                  // warp 0 consumer; 4, 8 and 11 idle
+constexpr int kBlk = 64;        // entries per block: two per lane while they are staged
+constexpr int kProducers = 6;
+constexpr int kSlots = 6;       // ring slots: block g is in slot g % kSlots
+constexpr int kWarps = 8;       // warp 0 the consumer, warp 4 idle
 constexpr int kThreads = 32 * kWarps;
-constexpr unsigned kSpinLimit = 1u << 22;   // polls of a bounded wait (a few seconds at most)
-static_assert(kStages % kProducers == 0, "a slot is always refilled by the same producer warp");
-static_assert(kStage == 64, "each producer lane holds two entries' index and value");
+constexpr int kGrp = 8;         // entries read into registers together
+constexpr unsigned kSpinLimit = 1u << 22;  // polls of a producer's wait
+constexpr unsigned kAll = 0xffffffffu;
+static_assert(kSlots % kProducers == 0, "a slot is always refilled by the same producer warp");
 
-template <typename T>
-struct Layout {
-    static constexpr int kSlice = kCols * static_cast<int>(sizeof(T));  // B bytes per entry
-    static constexpr int kRing = kStages * kStage * kSlice;
-    static constexpr int kVals = kStages * kStage * 4;                  // values as fp32
-    static constexpr int kMasks = kStages * 8;  // row-pair mode: the stage's include bits
-    static constexpr int kBytes = kRing + kVals + kMasks + 2 * kStages * 4 + 16;
-};
+constexpr int kSlotBytes = kBlk * 128;  // [kBlk / 4][32 lanes][4 entries] words
+constexpr int kRing = kSlots * kSlotBytes;
+constexpr int kVals = kSlots * kBlk * 4;
+constexpr int kSmem = kRing + kVals + 2 * kSlots * 8 + 16;
 
-// producer index (0-7) of a warp, or -1 for the consumer and the idle warps
+// producer index (0-5) of a warp, or -1 for the consumer and the idle warp
 __device__ __forceinline__ int producer_of(int warp) {
-    return (warp & 3) != 0 && warp <= 10 ? warp - 1 - (warp >> 2) : -1;
+    return (warp & 3) != 0 ? warp - 1 - (warp >> 2) : -1;
 }
-
-__device__ __forceinline__ float to_f32(float v) { return v; }
-__device__ __forceinline__ float to_f32(uint16_t v) { return bf16_to_f32(v); }
 
 __device__ __forceinline__ uint32_t smem_u32(const void *p) {
     return static_cast<uint32_t>(__cvta_generic_to_shared(p));
 }
-
-__device__ __forceinline__ int ld_acquire(uint32_t a) {
-    int v;
-    asm volatile("ld.acquire.cta.shared::cta.b32 %0, [%1];" : "=r"(v) : "r"(a) : "memory");
-    return v;
+__device__ __forceinline__ void mbar_init(uint32_t bar, unsigned count) {
+    asm volatile("mbarrier.init.shared::cta.b64 [%0], %1;" ::"r"(bar), "r"(count) : "memory");
 }
-__device__ __forceinline__ void st_release(uint32_t a, int v) {
-    asm volatile("st.release.cta.shared::cta.b32 [%0], %1;" ::"r"(a), "r"(v) : "memory");
+__device__ __forceinline__ void mbar_arrive(uint32_t bar) {
+    asm volatile("mbarrier.arrive.shared::cta.b64 _, [%0];" ::"r"(bar) : "memory");
 }
-// Bounded wait until the flag at `a` reaches `target`; false when `limit` polls pass or the
-// other role has given up. `nap` > 0 sleeps that many ns between polls (producers, which are
-// ahead and must not take issue slots from the consumer).
-__device__ __forceinline__ bool wait_seq(uint32_t a, int target, unsigned limit,
-                                         const volatile int *abort_flag, unsigned nap = 0) {
+// Whether the barrier's phase of this parity has completed (waits a short, bounded time).
+__device__ __forceinline__ bool mbar_try(uint32_t bar, unsigned parity) {
+    unsigned ok;
+    asm volatile(
+        "{\n\t.reg .pred p;\n\t"
+        "mbarrier.try_wait.parity.shared::cta.b64 p, [%1], %2;\n\t"
+        "selp.u32 %0, 1, 0, p;\n\t}"
+        : "=r"(ok)
+        : "r"(bar), "r"(parity)
+        : "memory");
+    return ok != 0;
+}
+// The same without waiting.
+__device__ __forceinline__ bool mbar_test(uint32_t bar, unsigned parity) {
+    unsigned ok;
+    asm volatile(
+        "{\n\t.reg .pred p;\n\t"
+        "mbarrier.test_wait.parity.shared::cta.b64 p, [%1], %2;\n\t"
+        "selp.u32 %0, 1, 0, p;\n\t}"
+        : "=r"(ok)
+        : "r"(bar), "r"(parity)
+        : "memory");
+    return ok != 0;
+}
+// Bounded wait for a barrier's phase; false when `limit` polls pass or the other role gave up.
+__device__ __forceinline__ bool mbar_wait(uint32_t bar, unsigned parity, unsigned limit,
+                                          const volatile int *abort_flag) {
     for (unsigned i = 0; i < limit; ++i) {
-        if (ld_acquire(a) >= target) return true;
+        if (mbar_try(bar, parity)) return true;
         if (*abort_flag) return false;
-        if (nap) __nanosleep(nap);
     }
     return false;
 }
 
-// Two consecutive B columns of one entry from shared memory, as fp32.
-__device__ __forceinline__ float2 lds_pair(uint32_t a, float) {
-    float2 r;
-    asm volatile("ld.shared.v2.f32 {%0, %1}, [%2];" : "=f"(r.x), "=f"(r.y) : "r"(a));
-    return r;
-}
-__device__ __forceinline__ float2 lds_pair(uint32_t a, uint16_t) {
-    uint32_t u;
-    asm volatile("ld.shared.u32 %0, [%1];" : "=r"(u) : "r"(a));
-    return make_float2(__uint_as_float(u << 16), __uint_as_float(u & 0xffff0000u));
-}
-__device__ __forceinline__ float4 lds_vals(uint32_t a) {
-    float4 r;
-    asm volatile("ld.shared.v4.f32 {%0, %1, %2, %3}, [%4];"
-                 : "=f"(r.x), "=f"(r.y), "=f"(r.z), "=f"(r.w)
-                 : "r"(a));
-    return r;
-}
-
-template <int GB>
-__device__ __forceinline__ void cp_async_zfill(uint32_t dst, const void *gmem, int src_bytes) {
-    if constexpr (GB == 16)
-        asm volatile("cp.async.cg.shared.global [%0], [%1], 16, %2;\n" ::"r"(dst), "l"(gmem),
-                     "r"(src_bytes)
-                     : "memory");
-    else
-        asm volatile("cp.async.ca.shared.global [%0], [%1], 4, %2;\n" ::"r"(dst), "l"(gmem),
-                     "r"(src_bytes)
-                     : "memory");
-}
-
-// The per-entry step of a chain: OP 0 the SpMM's fused multiply-add (acc = fma(b, v, acc)),
+// One chain step for each of a lane's columns, from the entry's 32-bit word of B (a float, or
+// two bf16) and its staged value: OP 0 the SpMM's fused multiply-add (acc = fma(b, v, acc)),
 // 1 the unweighted copy-sum (acc + b), 2 max from -inf (fmaxf(acc, v * b)), 3 the DGL max
 // (acc > v * b ? acc : v * b), 4 the fused multiply-add skipping zero values (the 1x4-blocked
-// layout's empty slots), 5 the fused multiply-add over the entries a row-pair unit includes
-// (the include mask is applied by the consumer); the max forms use b alone when the row has
-// no values.
+// layout's empty slots), 5 the fused multiply-add over the entries a row-pair unit includes. The
+// max forms find 1.0f as the value of an unweighted entry (x * 1.0f is x).
 template <int OP>
-__device__ __forceinline__ float step(float acc, float b, float v, bool weighted) {
-    if constexpr (OP == 0) return fmaf(b, v, acc);
-    if constexpr (OP == 1) return __fadd_rn(acc, b);
-    if constexpr (OP == 4) return v != 0.0f ? fmaf(b, v, acc) : acc;
-    if constexpr (OP == 5) return fmaf(b, v, acc);
-    const float x = weighted ? __fmul_rn(v, b) : b;
-    if constexpr (OP == 2) return fmaxf(acc, x);
-    return acc > x ? acc : x;
+__device__ __forceinline__ void step(float (&acc)[1], unsigned w, float v) {
+    const float b = __uint_as_float(w);
+    if constexpr (OP == 0 || OP == 5) acc[0] = fmaf(b, v, acc[0]);
+    if constexpr (OP == 1) acc[0] = __fadd_rn(acc[0], b);
+    if constexpr (OP == 2) acc[0] = fmaxf(acc[0], __fmul_rn(v, b));
+    if constexpr (OP == 3) {
+        const float x = __fmul_rn(v, b);
+        acc[0] = acc[0] > x ? acc[0] : x;
+    }
+    if constexpr (OP == 4) acc[0] = v != 0.0f ? fmaf(b, v, acc[0]) : acc[0];
+}
+template <int OP>
+__device__ __forceinline__ void step(float (&acc)[2], unsigned w, float v) {
+    fma_bf16x2(w, static_cast<unsigned short>(__float_as_uint(v)), acc[0], acc[1]);
+}
+// The staged form of a value: a float's bits, or a bf16's 16 bits in a word.
+__device__ __forceinline__ float staged(float v) { return v; }
+__device__ __forceinline__ float staged(uint16_t v) { return __uint_as_float(v); }
+
+// The word of a segment that consumer lane l holds.
+__device__ __forceinline__ int word_of(int l) { return l % 8 * 4 + l / 8; }
+
+__device__ __forceinline__ void prefetch_l2(const void *p) {
+    asm volatile("prefetch.global.L2 [%0];" ::"l"(p));
 }
 
-// T: storage type of val and B (float or uint16_t = bf16); GB: cp.async size in bytes; OP: the
+// How the rows of B can be read: 16 bytes at a time, 4 bytes, or (bf16) 2 bytes.
+enum Access { kVec, kWord, kHalf };
+
+// Loads of B, volatile: issued where they stand, all of a block before the wait for its slot.
+// A lane's word of one entry's segment (p: its first column): a float, or two bf16 (kHalf: with
+// two 2-byte loads).
+template <int ACC>
+__device__ __forceinline__ unsigned load_word(const void *p, bool second) {
+    unsigned v;
+    if constexpr (ACC != kHalf) {
+        asm volatile("ld.global.nc.u32 %0, [%1];" : "=r"(v) : "l"(p));
+    } else {
+        unsigned short lo, hi;
+        asm volatile("ld.global.nc.u16 %0, [%1];" : "=h"(lo) : "l"(p));
+        // a lane without a second column in the row reads its first again
+        asm volatile("ld.global.nc.u16 %0, [%1];" : "=h"(hi)
+                     : "l"(static_cast<const char *>(p) + (second ? 2 : 0)));
+        v = lo | static_cast<unsigned>(hi) << 16;
+    }
+    return v;
+}
+__device__ __forceinline__ void load_vec(const void *p, unsigned *b) {
+    asm volatile("ld.global.nc.v4.u32 {%0, %1, %2, %3}, [%4];"
+                 : "=r"(b[0]), "=r"(b[1]), "=r"(b[2]), "=r"(b[3])
+                 : "l"(p));
+}
+
+// kGrp entries of a block in the consumer's registers: this lane's words of B and the values.
+// The reads are volatile: they are issued where they stand, ahead of the steps of the group
+// before.
+struct Group {
+    unsigned b[kGrp];
+    float v[kGrp];
+    __device__ __forceinline__ void read(uint32_t bs, uint32_t vs, int grp) {
+#pragma unroll
+        for (int i = 0; i < kGrp; i += 4) {
+            asm volatile("ld.shared.v4.f32 {%0, %1, %2, %3}, [%4];"
+                         : "=f"(v[i]), "=f"(v[i + 1]), "=f"(v[i + 2]), "=f"(v[i + 3])
+                         : "r"(vs + 4 * (grp * kGrp + i)));
+            asm volatile("ld.shared.v4.b32 {%0, %1, %2, %3}, [%4];"
+                         : "=r"(b[i]), "=r"(b[i + 1]), "=r"(b[i + 2]), "=r"(b[i + 3])
+                         : "r"(bs + 128 * (grp * kGrp + i)));
+        }
+    }
+    template <int OP, int CPL>
+    __device__ __forceinline__ void steps(float (&acc)[CPL]) const {
+#pragma unroll
+        for (int i = 0; i < kGrp; ++i) step<OP>(acc, b[i], v[i]);
+    }
+};
+
+// T: storage type of val and B (float or uint16_t = bf16); ACC: how B is read; OP: the
 // chain step above (the steps other than 0 take fp32 only). pair_flag: the row-pair layout's
 // flags (OP 5 only).
-template <typename T, int GB, int OP>
-__global__ void __launch_bounds__(kThreads, 1)
+template <typename T, int ACC, int OP>
+__global__ void __launch_bounds__(kThreads, 2)
 spmm_long(int M, int K, int N, int nnz, const int *__restrict__ rowptr,
           const int *__restrict__ colind, const T *__restrict__ val, const T *__restrict__ B,
           long ldb, float *__restrict__ C, long ldc, float beta, unsigned *status,
           const int *__restrict__ list, unsigned *counters, uint16_t *__restrict__ C16,
           bool relu, unsigned spin_limit, const uint8_t *__restrict__ pair_flag) {
-    using Lay = Layout<T>;
-    constexpr int kSlice = Lay::kSlice;
-    constexpr int kEsz = static_cast<int>(sizeof(T));
-    constexpr unsigned kAll = 0xffffffffu;
+    constexpr int CPL = 4 / static_cast<int>(sizeof(T));  // columns per lane
+    constexpr int kCols = 32 * CPL;                       // columns per slice
     extern __shared__ __align__(1024) unsigned char smem[];
-    unsigned char *ring = smem;                                  // [kStages][kStage][kSlice]
-    float *vals = reinterpret_cast<float *>(smem + Lay::kRing);  // [kStages][kStage]
-    unsigned long long *masks = reinterpret_cast<unsigned long long *>(smem + Lay::kRing + Lay::kVals);
-    int *full_seq = reinterpret_cast<int *>(smem + Lay::kRing + Lay::kVals + Lay::kMasks);  // stage filled + 1
-    int *empty_seq = full_seq + kStages;                                       // stage consumed + 1
-    volatile int *abort_flag = reinterpret_cast<volatile int *>(empty_seq + kStages);
+    unsigned char *ring = smem;                              // [kSlots][kSlotBytes]
+    float *vals = reinterpret_cast<float *>(smem + kRing);   // [kSlots][kBlk]
+    // per slot: filled (one arrival by its producer), consumed (one by the consumer)
+    const uint32_t full_bar = smem_u32(smem + kRing + kVals), empty_bar = full_bar + 8 * kSlots;
+    volatile int *abort_flag =
+        reinterpret_cast<volatile int *>(smem + kRing + kVals + 2 * kSlots * 8);
 
     // launched as a programmatic dependent of the row-split kernel: wait for it to finish
     // (and its list writes to be visible) before reading the list
@@ -178,221 +235,294 @@ spmm_long(int M, int K, int N, int nnz, const int *__restrict__ rowptr,
     const int n_long = static_cast<int>(min(*reinterpret_cast<volatile unsigned *>(counters), cap));
     const int n_huge =
         static_cast<int>(min(*reinterpret_cast<volatile unsigned *>(counters + 2), cap));
+    if (n_long + n_huge == 0) return;  // nothing listed: every CTA sees that, nothing to reset
+    if (tid < 2 * kSlots) mbar_init(full_bar + 8 * tid, 1);
+    if (tid == 0) *abort_flag = 0;
+    __syncthreads();
+
     // row-pair mode: a listed item is a pair's even row; each pair gives two rows' units
     constexpr int kRowsPerItem = OP == 5 ? 2 : 1;
     const int n_slices = static_cast<int>(ceil_div(N, kCols)) * kRowsPerItem;
     const long units_huge = static_cast<long>(n_huge) * n_slices;
     const long units = units_huge + static_cast<long>(n_long) * n_slices;
+    // This CTA's units. The huge rows' units (listed from the end) come first. Where they are
+    // fewer than half of the CTAs, each has a CTA of its own and the others share the rest:
+    // the longest chain is the call's critical path, and nothing is queued behind it.
+    long u_first = blockIdx.x, u_step = gridDim.x, u_end = units;
+    if (units_huge > 0 && 2 * units_huge <= gridDim.x) {
+        if (blockIdx.x < units_huge)
+            u_end = units_huge;
+        else
+            u_step = gridDim.x - units_huge;
+    }
     const int pw = producer_of(warp);
+    const bool weighted = val != nullptr;
+    unsigned seq = 0;  // blocks of the CTA's stream before the current batch of units
+    bool dead = warp != 0 && pw < 0;  // the idle warp leaves at once
 
-    // work units (row, column slice): the huge rows (listed from the end) first, the slices of
-    // one row on consecutive CTAs
-    for (long u = blockIdx.x; u < units; u += gridDim.x) {
-        const bool huge = u < units_huge;
-        const long v = huge ? u : u - units_huge;
-        const int item = static_cast<int>(v / n_slices);
-        const int sub_unit = static_cast<int>(v - static_cast<long>(item) * n_slices);
-        const int which = sub_unit % kRowsPerItem;   // row-pair mode: 0 the even row, 1 the odd
-        const int slice0 = sub_unit / kRowsPerItem * kCols;
-        const int w = min(kCols, N - slice0);        // columns of this slice
-        const int pieces = w * kEsz / GB;            // copy pieces per entry
-        const int r0 = huge ? list[M - 1 - item] : list[item];
-        const int r = r0 + which;                    // the output row
-        if (r0 < 0 || r >= M) continue;
-        int lo, hi;
-        row_range(rowptr, r0, nnz, status, lo, hi);
-        // Row-pair mode: the even row chains over its segment's unflagged entries (all of them
-        // when it has no partner); the odd row over the even segment's flagged entries, then
-        // over its own segment (entries at positions L1.. map to [lo1, hi1)).
-        int L1 = hi - lo, lo1 = 0, hi1 = 0;
-        const bool partner = OP == 5 && r0 + 1 < M;
-        if (OP == 5 && which == 1) row_range(rowptr, r0 + 1, nnz, status, lo1, hi1);
-        const int L = L1 + (hi1 - lo1);
-        const int n_stages = static_cast<int>(ceil_div(L, kStage));
-
-        if (tid == 0) {
-            for (int s = 0; s < kStages; ++s) {
-                full_seq[s] = 0;
-                empty_seq[s] = 0;
+    // the units in batches of 32, one per lane; every warp walks the same stream
+    for (long ub = u_first; ub < u_end && !dead; ub += 32 * u_step) {
+        const long u = ub + lane * u_step;
+        int m_r = -1, m_lo = 0, m_lo1 = 0, m_L1 = 0, m_L = 0, m_slice = 0, m_nb = 0;
+        if (u < u_end) {
+            const bool huge = u < units_huge;
+            const long v = huge ? u : u - units_huge;
+            const int item = static_cast<int>(v / n_slices);
+            const int sub = static_cast<int>(v - static_cast<long>(item) * n_slices);
+            const int which = sub % kRowsPerItem;  // row-pair mode: 0 the even row, 1 the odd
+            const int r0 = huge ? list[M - 1 - item] : list[item];
+            if (r0 >= 0 && r0 + which < M) {
+                // Row-pair mode: the even row chains over its segment's unflagged entries (all
+                // of them when it has no partner); the odd row over the even segment's flagged
+                // entries, then over its own segment (entries at positions L1.. map to lo1..).
+                int hi, hi1 = 0;
+                row_range(rowptr, r0, nnz, status, m_lo, hi);
+                if (OP == 5 && which == 1) row_range(rowptr, r0 + 1, nnz, status, m_lo1, hi1);
+                m_r = r0 + which;
+                m_L1 = hi - m_lo;
+                m_L = m_L1 + (hi1 - m_lo1);
+                m_slice = sub / kRowsPerItem * kCols;
+                m_nb = max(1, static_cast<int>(ceil_div(m_L, kBlk)));
             }
-            *abort_flag = 0;
         }
-        __syncthreads();
+        int incl = m_nb;  // blocks of the batch's units up to and with this lane's
+#pragma unroll
+        for (int o = 1; o < 32; o <<= 1) {
+            const int y = __shfl_up_sync(kAll, incl, o);
+            if (lane >= o) incl += y;
+        }
+        const int n_units = static_cast<int>(min(32ll, ceil_div(u_end - ub, u_step)));
+        for (int j = 0; j < n_units && !dead; ++j) {
+            const int nb = __shfl_sync(kAll, m_nb, j);
+            if (nb == 0) continue;  // a malformed list entry
+            const unsigned base = seq + static_cast<unsigned>(__shfl_sync(kAll, incl, j) - nb);
+            const int L = __shfl_sync(kAll, m_L, j);
+            const int r = __shfl_sync(kAll, m_r, j);
+            const int slice0 = __shfl_sync(kAll, m_slice, j);
+            const int w = min(kCols, N - slice0);  // columns of this slice
 
-        constexpr float kInit = OP == 2 ? -INFINITY : OP == 3 ? -10000.0f : 0.0f;
-        const bool weighted = val != nullptr;
-        float acc0 = kInit, acc1 = kInit;
-        const int c0 = 2 * lane;  // this lane's first column within the slice
-        float *crow = C + static_cast<long>(r) * ldc + slice0;  // r: this unit's output row
-        if (warp == 0) {
-            // ---- consumer: the chains of columns c0 and c0 + 1 ----
-            if (beta != 0.0f) {
-                if (c0 < w) acc0 = crow[c0] * beta;
-                if (c0 + 1 < w) acc1 = crow[c0 + 1] * beta;
-            }
-            for (int s = 0; s < n_stages; ++s) {
-                const int slot = s % kStages;
-                const bool ok = __all_sync(kAll, wait_seq(smem_u32(full_seq + slot), s + 1,
-                                                          spin_limit, abort_flag));
-                if (!ok) {
-                    if (lane == 0) {
-                        flag(status, kFlagTimeout);
-                        *abort_flag = 1;
+            if (warp == 0) {
+                // ---- consumer: the chains of columns c0 .. c0 + CPL - 1 of the slice ----
+                constexpr float kInit = OP == 2 ? -INFINITY : OP == 3 ? -10000.0f : 0.0f;
+                const int c0 = CPL * word_of(lane);
+                const long out = static_cast<long>(r) * ldc + slice0 + c0;
+                float acc[CPL];
+#pragma unroll
+                for (int c = 0; c < CPL; ++c)
+                    acc[c] = beta != 0.0f && c0 + c < w ? C[out + c] * beta : kInit;
+                auto full_of = [&](unsigned g) { return full_bar + 8 * (g % kSlots); };
+                auto wait_full = [&](unsigned g) {  // block g of the stream is in its slot
+                    const bool ok = __all_sync(
+                        kAll, mbar_wait(full_of(g), g / kSlots & 1, spin_limit, abort_flag));
+                    if (!ok) {
+                        if (lane == 0) {
+                            flag(status, kFlagTimeout);
+                            *abort_flag = 1;
+                        }
+                        dead = true;
                     }
-                    break;
-                }
-                const int n = min(kStage, L - s * kStage);
-                const uint32_t bs = smem_u32(ring + slot * kStage * kSlice) + c0 * kEsz;
-                const uint32_t vs = smem_u32(vals + slot * kStage);
-                // row-pair mode: entry j of the stage counts when bit j is set
-                const unsigned long long mask = OP == 5 ? masks[slot] : ~0ull;
-                auto st = [&](float acc, float b, float x, int j) {
-                    if constexpr (OP == 5) return ((mask >> j) & 1ull) ? fmaf(b, x, acc) : acc;
-                    return step<OP>(acc, b, x, weighted);
+                    return ok;
                 };
-                if (n == kStage) {
+                auto release = [&](unsigned g) {  // its slot can be refilled
+                    __syncwarp();
+                    if (lane == 0) mbar_arrive(empty_bar + 8 * (g % kSlots));
+                };
+                auto b_of = [&](unsigned g) { return smem_u32(ring) + g % kSlots * kSlotBytes + 16 * lane; };
+                auto v_of = [&](unsigned g) { return smem_u32(vals) + g % kSlots * (kBlk * 4); };
+                const int nfull = L / kBlk;  // whole blocks
+                unsigned g = base;
+                if (nfull > 0 && wait_full(g)) {
+                    uint32_t bs = b_of(g), vs = v_of(g);
+                    constexpr int kG = kBlk / kGrp;  // groups per block, a multiple of four
+                    Group q[4];  // three groups are read ahead of the one that runs
+                    q[0].read(bs, vs, 0);
+                    q[1].read(bs, vs, 1);
+                    q[2].read(bs, vs, 2);
+#pragma unroll 1
+                    for (int t = 0; t < nfull; ++t, ++g) {
+                        const bool more = t + 1 < nfull;
+                        const bool ready = more && mbar_test(full_of(g + 1), (g + 1) / kSlots & 1);
 #pragma unroll
-                    for (int q = 0; q < kStage; q += 16) {
-                        float2 b[16];
-                        float4 v[4];
-#pragma unroll
-                        for (int i = 0; i < 16; ++i) b[i] = lds_pair(bs + (q + i) * kSlice, T());
-#pragma unroll
-                        for (int i = 0; i < 4; ++i) v[i] = lds_vals(vs + (q + 4 * i) * 4);
-#pragma unroll
-                        for (int i = 0; i < 4; ++i) {
-                            const int j = q + 4 * i;
-                            acc0 = st(acc0, b[4 * i].x, v[i].x, j);
-                            acc1 = st(acc1, b[4 * i].y, v[i].x, j);
-                            acc0 = st(acc0, b[4 * i + 1].x, v[i].y, j + 1);
-                            acc1 = st(acc1, b[4 * i + 1].y, v[i].y, j + 1);
-                            acc0 = st(acc0, b[4 * i + 2].x, v[i].z, j + 2);
-                            acc1 = st(acc1, b[4 * i + 2].y, v[i].z, j + 2);
-                            acc0 = st(acc0, b[4 * i + 3].x, v[i].w, j + 3);
-                            acc1 = st(acc1, b[4 * i + 3].y, v[i].w, j + 3);
+                        for (int i = 0; i < kG; ++i) {
+                            if (i == kG - 3) {
+                                if (more && !__all_sync(kAll, ready) && !wait_full(g + 1)) break;
+                                if (more) bs = b_of(g + 1), vs = v_of(g + 1);
+                            }
+                            // (past the last whole block: reads of it again, not used)
+                            q[(i + 3) % 4].read(bs, vs, (i + 3) % kG);
+                            q[i % 4].template steps<OP>(acc);
                         }
-                    }
-                } else {
-                    for (int j = 0; j < n; ++j) {
-                        const float2 b = lds_pair(bs + j * kSlice, T());
-                        const float x = vals[slot * kStage + j];
-                        acc0 = st(acc0, b.x, x, j);
-                        acc1 = st(acc1, b.y, x, j);
+                        if (dead) break;
+                        release(g);
                     }
                 }
-                __syncwarp();
-                if (lane == 0) st_release(smem_u32(empty_seq + slot), s + 1);
-            }
-        } else if (pw >= 0) {
-            // ---- producer pw: stages pw, pw + kProducers, ... (all in slot pw % kStages) ----
-            const int sub = lane >> 3, pl = lane & 7;  // entry of a group of four, lane in it
-            // column index and value of this lane's entries (lane, lane + 32) of stage st
-            // entry position e of the unit -> index in the arrays, and whether it counts
-            // (row-pair mode; every entry counts otherwise)
-            auto entry = [&](int e, int &idx, int &inc) {
-                idx = lo + e;
-                inc = 1;
-                if constexpr (OP == 5) {
-                    if (e >= L1) {
-                        idx = lo1 + (e - L1);
-                    } else if (partner) {
-                        inc = (__ldg(pair_flag + idx) != 0) == (which == 1);
+                // the last, partial block: its groups that hold an entry
+                if (g != base + nb && !dead && wait_full(g)) {
+                    const int n = L - nfull * kBlk;
+#pragma unroll 1
+                    for (int i = 0; i * kGrp < n; ++i) {
+                        Group p;
+                        p.read(b_of(g), v_of(g), i);
+                        p.template steps<OP>(acc);
                     }
+                    release(g);
                 }
-            };
-            auto load = [&](int st, int &k0, int &k1, float &x0, float &x1, int &f0, int &f1) {
-                k0 = k1 = 0;
-                x0 = x1 = 0.0f;
-                f0 = f1 = 0;
-                const int e0 = st * kStage + lane, e1 = e0 + 32;
-                int i0, i1;
-                if (st < n_stages && e0 < L) {
-                    entry(e0, i0, f0);
-                    k0 = ld_stream(colind + i0);
-                    x0 = weighted ? to_f32(ld_stream(val + i0)) : 1.0f;
-                }
-                if (st < n_stages && e1 < L) {
-                    entry(e1, i1, f1);
-                    k1 = ld_stream(colind + i1);
-                    x1 = weighted ? to_f32(ld_stream(val + i1)) : 1.0f;
-                }
-            };
-            int k0, k1, f0, f1;
-            float x0, x1;
-            load(pw, k0, k1, x0, x1, f0, f1);
-            for (int s = pw; s < n_stages; s += kProducers) {
-                const int slot = s % kStages;
-                if (s >= kStages) {  // the consumer is done with stage s - kStages
-                    int ok = 1;
-                    if (lane == 0)
-                        ok = wait_seq(smem_u32(empty_seq + slot), s - kStages + 1, kSpinLimit,
-                                      abort_flag, 64);
-                    if (!__shfl_sync(kAll, ok, 0)) break;
-                }
-                int nk0, nk1, nf0, nf1;
-                float nx0, nx1;
-                load(s + kProducers, nk0, nk1, nx0, nx1, nf0, nf1);  // the next turn's, in flight meanwhile
-                vals[slot * kStage + lane] = x0;
-                vals[slot * kStage + lane + 32] = x1;
-                if constexpr (OP == 5) {
-                    const unsigned long long m =
-                        __ballot_sync(kAll, f0) | (static_cast<unsigned long long>(__ballot_sync(kAll, f1)) << 32);
-                    if (lane == 0) masks[slot] = m;
-                }
-                const uint32_t dst0 = smem_u32(ring + slot * kStage * kSlice);
-#pragma unroll 4
-                for (int g = 0; g < kStage / 4; ++g) {
-                    const int j = 4 * g + sub;
-                    int k = __shfl_sync(kAll, g < 8 ? k0 : k1, j & 31);
-                    // OP 4: an empty slot (value 0) may point past K; only a filled one is bad.
-                    // OP 5: an entry the unit leaves out is neither checked nor copied.
-                    bool filled = true;
-                    if constexpr (OP == 4) filled = __shfl_sync(kAll, g < 8 ? x0 : x1, j & 31) != 0.0f;
-                    if constexpr (OP == 5) filled = __shfl_sync(kAll, g < 8 ? f0 : f1, j & 31) != 0;
-                    if (s * kStage + j < L && (OP != 5 || filled)) {
-                        const bool bad = static_cast<unsigned>(k) >= static_cast<unsigned>(K);
-                        if (bad) {
-                            if (filled) flag(status, kFlagBadColind);
-                            k = 0;
-                        }
-                        const unsigned char *src = reinterpret_cast<const unsigned char *>(
-                            B + static_cast<long>(k) * ldb + slice0);
-                        const uint32_t dst = dst0 + j * kSlice;
+                if (!dead) {
 #pragma unroll
-                        for (int q = 0; q < kSlice / GB / 8; ++q) {
-                            const int piece = pl + 8 * q;
-                            if (piece < pieces)
-                                cp_async_zfill<GB>(dst + piece * GB, src + piece * GB, bad ? 0 : GB);
-                        }
+                    for (int c = 0; c < CPL; ++c) {
+                        if (c0 + c >= w) continue;
+                        if (C16)
+                            C16[out + c] = f32_to_bf16(relu_if(acc[c], relu));
+                        else
+                            C[out + c] = acc[c];
                     }
                 }
-                // the slot is full once every lane's copies have landed
-                asm volatile("cp.async.commit_group;\n" ::: "memory");
-                asm volatile("cp.async.wait_group 0;\n" ::: "memory");
-                __syncwarp();
-                if (lane == 0) st_release(smem_u32(full_seq + slot), s + 1);
-                k0 = nk0;
-                k1 = nk1;
-                x0 = nx0;
-                x1 = nx1;
-                f0 = nf0;
-                f1 = nf1;
-            }
-            asm volatile("cp.async.wait_all;\n" ::: "memory");
-            __syncwarp();
-        }
-        __syncthreads();
-        if (warp == 0 && !*abort_flag) {
-            if (C16) {
-                uint16_t *orow = C16 + static_cast<long>(r) * ldc + slice0;
-                if (c0 < w) orow[c0] = f32_to_bf16(relu_if(acc0, relu));
-                if (c0 + 1 < w) orow[c0 + 1] = f32_to_bf16(relu_if(acc1, relu));
             } else {
-                if (c0 < w) crow[c0] = acc0;
-                if (c0 + 1 < w) crow[c0 + 1] = acc1;
+                // ---- producer pw: the blocks g of the stream with g % kProducers == pw ----
+                const int t0 = static_cast<int>((kProducers + pw - base % kProducers) % kProducers);
+                if (t0 >= nb) continue;
+                const int lo = __shfl_sync(kAll, m_lo, j);
+                int lo1 = 0, L1 = L, which = 0;
+                bool partner = false;
+                if constexpr (OP == 5) {
+                    lo1 = __shfl_sync(kAll, m_lo1, j);
+                    L1 = __shfl_sync(kAll, m_L1, j);
+                    which = r & 1;  // pairs start at even rows
+                    partner = (r | 1) < M;
+                }
+                // this lane's words of a segment (a lane past the slice repeats one in range):
+                // four of every fourth entry (kVec), or its consumer lane's one
+                const int words = static_cast<int>(ceil_div(w, CPL));
+                const int wd = ACC == kVec ? min(lane % 8 * 4, words - 4) : min(word_of(lane), words - 1);
+                const int sub = lane / 8;
+                const bool second = CPL * wd + 1 < w;
+                const T *bcol = B + slice0 + CPL * wd;
+                constexpr unsigned kSkipWord = sizeof(T) == 4 ? 0x80000000u : 0x80008000u;  // -0.0
+                const float one = sizeof(T) == 4 ? 1.0f : __uint_as_float(0x3f80u);  // staged 1
+                // column index (-1: the position adds nothing, -2: out of range) and value of
+                // this lane's entries of block t
+                auto load = [&](int t, int (&k)[2], float (&x)[2]) {
+#pragma unroll
+                    for (int h = 0; h < 2; ++h) {
+                        int e = t * kBlk + 32 * h + lane;
+                        k[h] = -1;
+                        x[h] = OP == 4 ? 0.0f : one;
+                        // the max steps: a position past the end repeats the last entry (which
+                        // leaves them as they are)
+                        if (OP == 2 || OP == 3) e = min(e, L - 1);
+                        if (t >= nb || e >= L || e < 0) continue;
+                        int idx = lo + e;
+                        if constexpr (OP == 5) {
+                            if (e >= L1)
+                                idx = lo1 + (e - L1);
+                            else if (partner && (__ldg(pair_flag + idx) != 0) != (which == 1))
+                                continue;  // the other row's: neither checked nor read
+                        }
+                        k[h] = ld_stream(colind + idx);
+                        if (weighted) x[h] = staged(ld_stream(val + idx));
+                        // OP 4: an empty slot (value 0) may point past K; only a filled one is bad
+                        if (OP == 4 && x[h] == 0.0f)
+                            k[h] = -1;
+                        else if (static_cast<unsigned>(k[h]) >= static_cast<unsigned>(K))
+                            k[h] = -2;
+                    }
+                };
+                int k[2];
+                float x[2];
+                load(t0, k, x);
+#pragma unroll 1
+                for (int t = t0; t < nb; t += kProducers) {
+                    const unsigned g = base + static_cast<unsigned>(t);
+                    const int slot = static_cast<int>(g % kSlots);
+                    if (k[0] == -2 || k[1] == -2) flag(status, kFlagBadColind);
+                    unsigned char *dst = ring + slot * kSlotBytes;
+                    // the consumer is done with block g - kSlots
+                    auto slot_free = [&] {
+                        if (g < kSlots) return true;
+                        return static_cast<bool>(
+                            __all_sync(kAll, mbar_wait(empty_bar + 8 * slot, (g / kSlots - 1) & 1,
+                                                       kSpinLimit, abort_flag)));
+                    };
+                    int nk[2];
+                    float nx[2];
+                    if constexpr (ACC == kVec) {
+                        int kk[kBlk / 4];
+                        unsigned b[kBlk];
+#pragma unroll
+                        for (int i = 0; i < kBlk / 4; ++i)
+                            kk[i] = __shfl_sync(kAll, k[i / 8], i % 8 * 4 + sub);
+                        if (__all_sync(kAll, k[0] >= 0 && k[1] >= 0)) {
+#pragma unroll
+                            for (int i = 0; i < kBlk / 4; ++i) load_vec(bcol + kk[i] * ldb, b + 4 * i);
+                        } else {
+#pragma unroll
+                            for (int i = 0; i < kBlk / 4; ++i) {
+#pragma unroll
+                                for (int u = 0; u < 4; ++u) b[4 * i + u] = kk[i] == -1 ? kSkipWord : 0u;
+                                if (kk[i] >= 0) load_vec(bcol + kk[i] * ldb, b + 4 * i);
+                            }
+                        }
+                        load(t + kProducers, nk, nx);  // the next turn's, in flight meanwhile
+                        if (!slot_free()) {
+                            dead = true;
+                            break;
+                        }
+#pragma unroll
+                        for (int i = 0; i < kBlk; ++i)  // word 4 * (lane % 8) + i % 4 of an entry
+                            *reinterpret_cast<unsigned *>(dst + 128 * i + lane % 8 * 16 + sub * 4) =
+                                b[i];
+                    } else {
+                        // one word per lane and entry: in two halves, which the registers hold
+#pragma unroll 1
+                        for (int h = 0; h < 2 && !dead; ++h) {
+                            unsigned b[kBlk / 2];
+                            const int kh = h ? k[1] : k[0];
+                            const bool clean = __all_sync(kAll, kh >= 0);
+#pragma unroll
+                            for (int i0 = 0; i0 < kBlk / 2; i0 += 8) {
+                                int kk[8];
+#pragma unroll
+                                for (int i = 0; i < 8; ++i) kk[i] = __shfl_sync(kAll, kh, i0 + i);
+                                if (clean) {
+#pragma unroll
+                                    for (int i = 0; i < 8; ++i)
+                                        b[i0 + i] = load_word<ACC>(bcol + kk[i] * ldb, second);
+                                } else {
+#pragma unroll
+                                    for (int i = 0; i < 8; ++i) {
+                                        b[i0 + i] = kk[i] == -1 ? kSkipWord : 0u;
+                                        if (kk[i] >= 0)
+                                            b[i0 + i] = load_word<ACC>(bcol + kk[i] * ldb, second);
+                                    }
+                                }
+                            }
+                            if (h == 0) {
+                                load(t + kProducers, nk, nx);
+                                dead = !slot_free();
+                                if (dead) break;
+                            }
+#pragma unroll
+                            for (int i = 0; i < kBlk / 2; i += 4)
+                                *reinterpret_cast<uint4 *>(dst + 128 * (32 * h + i) + 16 * lane) =
+                                    make_uint4(b[i], b[i + 1], b[i + 2], b[i + 3]);
+                        }
+                        if (dead) break;
+                    }
+                    vals[slot * kBlk + lane] = x[0];
+                    vals[slot * kBlk + 32 + lane] = x[1];
+                    __syncwarp();
+                    if (lane == 0) mbar_arrive(full_bar + 8 * slot);
+#pragma unroll
+                    for (int h = 0; h < 2; ++h) {
+                        k[h] = nk[h];
+                        x[h] = nx[h];
+                        // the next turn's segments on their way into L2
+                        if (k[h] >= 0) prefetch_l2(B + slice0 + k[h] * ldb);
+                    }
+                }
             }
         }
-        __syncthreads();  // shared memory and flags are reused by the next unit
+        seq += static_cast<unsigned>(__shfl_sync(kAll, incl, 31));
     }
 
     // the last CTA out resets the list counters and the done counter for the next call
@@ -409,24 +539,24 @@ spmm_long(int M, int K, int N, int nnz, const int *__restrict__ rowptr,
     }
 }
 
-template <typename T, int GB, int OP = 0>
+template <typename T, int ACC, int OP = 0>
 as_status launch(as_ctx *ctx, const SpmmArgs &a, const int *list, cudaStream_t s,
                  const uint8_t *pair_flag = nullptr) {
-    auto k = spmm_long<T, GB, OP>;
-    constexpr int kBytes = Layout<T>::kBytes;
+    auto k = spmm_long<T, ACC, OP>;
     static int per_sm[64] = {};  // resident CTAs per multiprocessor, per device
     const int dev = ctx->device;
     if (dev < 0 || dev >= 64) return fail(AS_ERR_INVALID_VALUE, "spmm long rows: device index");
     if (!per_sm[dev]) {
-        cudaError_t e = cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, kBytes);
+        cudaError_t e = cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, kSmem);
         if (e != cudaSuccess) return check_cuda(e, "spmm long rows: shared memory attribute");
         int n = 0;
-        e = cudaOccupancyMaxActiveBlocksPerMultiprocessor(&n, k, kThreads, kBytes);
+        e = cudaOccupancyMaxActiveBlocksPerMultiprocessor(&n, k, kThreads, kSmem);
         if (e != cudaSuccess) return check_cuda(e, "spmm long rows: occupancy");
         per_sm[dev] = std::max(1, n);
     }
     // one wave of CTAs striding over the (row, slice) units
-    const long max_units = static_cast<long>(a.M) * ceil_div(a.N, kCols) * (OP == 5 ? 2 : 1);
+    const long max_units = static_cast<long>(a.M) * ceil_div(a.N, 128 / static_cast<int>(sizeof(T))) *
+                           (OP == 5 ? 2 : 1);
     dim3 grid(static_cast<unsigned>(
         std::max(1L, std::min(max_units, static_cast<long>(per_sm[dev]) * ctx->sms))));
     // programmatic dependent launch (outside stream capture): the CTAs are scheduled while
@@ -436,7 +566,7 @@ as_status launch(as_ctx *ctx, const SpmmArgs &a, const int *list, cudaStream_t s
     cudaLaunchConfig_t cfg = {};
     cfg.gridDim = grid;
     cfg.blockDim = dim3(kThreads);
-    cfg.dynamicSmemBytes = kBytes;
+    cfg.dynamicSmemBytes = kSmem;
     cfg.stream = s;
     cudaLaunchAttribute attr[1];
     attr[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
@@ -453,33 +583,30 @@ as_status launch(as_ctx *ctx, const SpmmArgs &a, const int *list, cudaStream_t s
 
 }  // namespace
 
-int spmm_long_granule(int dtype, int N, long ldb, const void *B) {
-    const int esz = dtype == 0 ? 4 : 2;
-    const uintptr_t pb = reinterpret_cast<uintptr_t>(B);
-    if ((static_cast<long>(N) * esz) % 16 == 0 && (ldb * esz) % 16 == 0 && pb % 16 == 0) return 16;
-    if ((static_cast<long>(N) * esz) % 4 == 0 && (ldb * esz) % 4 == 0 && pb % 4 == 0) return 4;
-    return 0;
-}
-
-as_status spmm_long_launch(as_ctx *ctx, int dtype, int granule, const SpmmArgs &a,
-                           const int *list, cudaStream_t s, int op, const uint8_t *pair_flag) {
-    if (op != 0) {  // the reductions and the 1x4-blocked layout: fp32
-        if (dtype != 0) return fail(AS_ERR_UNSUPPORTED, "spmm long rows: this step takes fp32");
-        switch (op) {
-            case 1: return granule == 16 ? launch<float, 16, 1>(ctx, a, list, s) : launch<float, 4, 1>(ctx, a, list, s);
-            case 2: return granule == 16 ? launch<float, 16, 2>(ctx, a, list, s) : launch<float, 4, 2>(ctx, a, list, s);
-            case 3: return granule == 16 ? launch<float, 16, 3>(ctx, a, list, s) : launch<float, 4, 3>(ctx, a, list, s);
-            case 4: return granule == 16 ? launch<float, 16, 4>(ctx, a, list, s) : launch<float, 4, 4>(ctx, a, list, s);
-            case 5:
-                if (!pair_flag) return fail(AS_ERR_INVALID_VALUE, "spmm long rows: row pairs need their flags");
-                return granule == 16 ? launch<float, 16, 5>(ctx, a, list, s, pair_flag)
-                                     : launch<float, 4, 5>(ctx, a, list, s, pair_flag);
-        }
-        return fail(AS_ERR_INVALID_VALUE, "spmm long rows: unknown reduction");
+as_status spmm_long_launch(as_ctx *ctx, int dtype, const SpmmArgs &a, const int *list,
+                           cudaStream_t s, int op, const uint8_t *pair_flag) {
+    if (dtype != 0 && op != 0)
+        return fail(AS_ERR_UNSUPPORTED, "spmm long rows: this step takes fp32");
+    if (op == 5 && !pair_flag)
+        return fail(AS_ERR_INVALID_VALUE, "spmm long rows: row pairs need their flags");
+    const long esz = dtype == 0 ? 4 : 2;
+    auto rows_of = [&](long bytes) {  // every row of B (and its last piece) in aligned pieces
+        return a.N * esz % bytes == 0 && a.ldb * esz % bytes == 0 &&
+               reinterpret_cast<uintptr_t>(a.B) % bytes == 0;
+    };
+    const bool vec = rows_of(16);
+    if (dtype != 0) {
+        if (vec) return launch<uint16_t, kVec>(ctx, a, list, s);
+        return rows_of(4) ? launch<uint16_t, kWord>(ctx, a, list, s)
+                          : launch<uint16_t, kHalf>(ctx, a, list, s);
     }
-    if (dtype == 0)
-        return granule == 16 ? launch<float, 16>(ctx, a, list, s) : launch<float, 4>(ctx, a, list, s);
-    return granule == 16 ? launch<uint16_t, 16>(ctx, a, list, s) : launch<uint16_t, 4>(ctx, a, list, s);
+#define AS_LONG_OP(O)                                                                        \
+    case O:                                                                                  \
+        return vec ? launch<float, kVec, O>(ctx, a, list, s, pair_flag)                      \
+                   : launch<float, kWord, O>(ctx, a, list, s, pair_flag);
+    switch (op) { AS_LONG_OP(0) AS_LONG_OP(1) AS_LONG_OP(2) AS_LONG_OP(3) AS_LONG_OP(4) AS_LONG_OP(5) }
+#undef AS_LONG_OP
+    return fail(AS_ERR_INVALID_VALUE, "spmm long rows: unknown reduction");
 }
 
 }  // namespace as

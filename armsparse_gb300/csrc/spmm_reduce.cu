@@ -10,7 +10,7 @@
 // in CSR order, so an empty row stays at -10000.
 //
 // One warp per row; each lane owns CPL vectors of E columns of the row's column tile (16-byte
-// loads where the layout allows, scalar otherwise). Rows with more than kLongRow entries are left to the long-row kernel (spmm_long.cu,
+// loads where the layout allows, scalar otherwise). Long rows (long_row_threshold) are left to the long-row kernel (spmm_long.cu,
 // launched next with the same reduction as its chain step), as in the row-split SpMM: a hub
 // row would otherwise keep one warp busy for the whole call.
 #include <limits.h>
@@ -139,17 +139,14 @@ as_status spmm_reduce_launch(as_ctx *ctx, int op, const SpmmArgs &a, cudaStream_
                            spmm_default_variant(0, a.M, a.K, a.N, a.nnz, a.ldb, a.ldc, a.B, a.C),
                            a, s);
     if (ceil_div(a.N, 128) > 65535) return fail(AS_ERR_UNSUPPORTED, "spmm reduce: N too large");
-    // rows longer than kLongRow entries go to the long-row kernel when its copies can serve
-    // the layout
+    // long rows go to the long-row kernel
     int thresh = INT_MAX;
     int *list = nullptr;
-    const int granule = a.nnz > kLongRow && a.M > 0 ? spmm_long_granule(0, a.N, a.ldb, a.B) : 0;
-    if (granule) {
-        void *p = nullptr;
-        as_status st = scratch(ctx, static_cast<size_t>(a.M) * sizeof(int), &p);
+    const int long_row = long_row_threshold(a.nnz, a.M);
+    if (a.nnz > long_row && a.M > 0) {
+        as_status st = scratch_list(ctx, a.M, s, &list);
         if (st != AS_OK) return st;
-        thresh = kLongRow;
-        list = static_cast<int *>(p);
+        if (list) thresh = long_row;
     }
     const bool vec = a.N % 4 == 0 && a.ldb % 4 == 0 && a.ldc % 4 == 0 &&
                      reinterpret_cast<uintptr_t>(a.B) % 16 == 0 &&
@@ -160,10 +157,10 @@ as_status spmm_reduce_launch(as_ctx *ctx, int op, const SpmmArgs &a, cudaStream_
     else w ? launch<2, true>(a, vec, thresh, list, cnt, s) : launch<2, false>(a, vec, thresh, list, cnt, s);
     ctx->launches++;
     as_status st = check_cuda(cudaGetLastError(), "spmm reduce launch");
-    if (st != AS_OK || !granule) return st;
+    if (st != AS_OK || !list) return st;
     // the long rows' chain step: the weighted sum is the SpMM's fused multiply-add
     const int step = op == 0 ? (w ? 0 : 1) : op == 1 ? 2 : 3;
-    st = spmm_long_launch(ctx, 0, granule, a, list, s, step);
+    st = spmm_long_launch(ctx, 0, a, list, s, step);
     if (st != AS_OK) cudaMemsetAsync(ctx->d_long, 0, 3 * sizeof(unsigned), s);
     return st;
 }

@@ -19,7 +19,7 @@
 // is ignored (the entry counts for its own row), and a flagged first entry of a segment reuses
 // a zero segment. A column index out of range is flagged and its entry skipped.
 //
-// Pairs with more than kLongRow entries are left to the long-row kernel (spmm_long.cu, its
+// Long pairs (long_row_threshold) are left to the long-row kernel (spmm_long.cu, its
 // row-pair step): a unit per row of the pair runs the same chain over the entries it includes,
 // each with its own column's B segment (identical to the reused one in a well-formed layout).
 #include <limits.h>
@@ -166,17 +166,14 @@ as_status spmm_rowpair_launch(as_ctx *ctx, const SpmmArgs &a, const uint8_t *fla
     const bool pairs = a.N % 2 == 0 && a.ldb % 2 == 0 && a.ldc % 2 == 0 && pb % 8 == 0 && pc % 8 == 0;
     if (ceil_div(a.N, wide ? 256 : pairs ? 64 : 32) > 65535)
         return fail(AS_ERR_UNSUPPORTED, "spmm rowpair: N too large");
-    // pairs longer than kLongRow entries go to the long-row kernel when its copies can serve
-    // the layout
+    // long pairs go to the long-row kernel
     int thresh = INT_MAX;
     int *list = nullptr;
-    const int granule = a.nnz > kLongRow && a.M > 0 ? spmm_long_granule(0, a.N, a.ldb, a.B) : 0;
-    if (granule) {
-        void *p = nullptr;
-        as_status st = scratch(ctx, static_cast<size_t>(a.M) * sizeof(int), &p);
+    const int long_pair = long_row_threshold(a.nnz, (static_cast<long>(a.M) + 1) / 2);
+    if (a.nnz > long_pair && a.M > 0) {
+        as_status st = scratch_list(ctx, a.M, s, &list);
         if (st != AS_OK) return st;
-        thresh = kLongRow;
-        list = static_cast<int *>(p);
+        if (list) thresh = long_pair;
     }
     // widest vectors the layout allows: float4 x 2 for wide B, float2, then scalars
     if (wide)
@@ -187,8 +184,8 @@ as_status spmm_rowpair_launch(as_ctx *ctx, const SpmmArgs &a, const uint8_t *fla
         launch<4, 1>(a, flag2, thresh, list, ctx->d_long, s);
     ctx->launches++;
     as_status st = check_cuda(cudaGetLastError(), "spmm rowpair launch");
-    if (st != AS_OK || !granule) return st;
-    st = spmm_long_launch(ctx, 0, granule, a, list, s, 5, flag2);
+    if (st != AS_OK || !list) return st;
+    st = spmm_long_launch(ctx, 0, a, list, s, 5, flag2);
     if (st != AS_OK) cudaMemsetAsync(ctx->d_long, 0, 3 * sizeof(unsigned), s);
     return st;
 }

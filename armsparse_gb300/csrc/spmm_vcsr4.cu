@@ -8,7 +8,7 @@
 // skipped (the layout cannot tell a stored zero from an empty slot), so every output is one
 // fused chain over the row's nonzero entries in column order: bit for bit the CSR SpMM of the
 // same matrix without stored zeros. The four rows of a block are adjacent in B, which the
-// gathers see as one run of 4 * ldb elements. Rows with more than kLongRow slots are left to
+// gathers see as one run of 4 * ldb elements. Long rows (long_row_threshold) are left to
 // the long-row kernel (spmm_long.cu, its zero-skipping step), as in the row-split SpMM.
 #include <limits.h>
 
@@ -118,16 +118,13 @@ as_status spmm_vcsr4_launch(as_ctx *ctx, int M, int K, int N, int nslots, const 
     const bool pairs = N % 2 == 0 && ldb % 2 == 0 && ldc % 2 == 0 && pb % 8 == 0 && pc % 8 == 0;
     if (ceil_div(N, wide ? 256 : pairs ? 64 : 32) > 65535)
         return fail(AS_ERR_UNSUPPORTED, "spmm vcsr4: N too large");
-    // rows longer than kLongRow slots go to the long-row kernel when its copies can serve the
-    // layout
+    // long rows go to the long-row kernel
     LongList lr{INT_MAX, nullptr, ctx->d_long};
-    const int granule = nslots > kLongRow && M > 0 ? spmm_long_granule(0, N, ldb, B) : 0;
-    if (granule) {
-        void *p = nullptr;
-        as_status st = scratch(ctx, static_cast<size_t>(M) * sizeof(int), &p);
+    const int long_row = long_row_threshold(nslots, M);
+    if (nslots > long_row && M > 0) {
+        as_status st = scratch_list(ctx, M, s, &lr.list);
         if (st != AS_OK) return st;
-        lr.thresh = kLongRow;
-        lr.list = static_cast<int *>(p);
+        if (lr.list) lr.thresh = long_row;
     }
     if (wide)
         launch<16, 2>(M, K, N, nslots, vrowptr, vcolind, vval, B, ldb, C, ldc, beta, ctx->d_status, lr, s);
@@ -137,9 +134,9 @@ as_status spmm_vcsr4_launch(as_ctx *ctx, int M, int K, int N, int nslots, const 
         launch<4, 1>(M, K, N, nslots, vrowptr, vcolind, vval, B, ldb, C, ldc, beta, ctx->d_status, lr, s);
     ctx->launches++;
     as_status st = check_cuda(cudaGetLastError(), "spmm vcsr4 launch");
-    if (st != AS_OK || !granule) return st;
+    if (st != AS_OK || !lr.list) return st;
     SpmmArgs a{M, K, N, nslots, vrowptr, vcolind, vval, B, ldb, C, ldc, beta, ctx->d_status};
-    st = spmm_long_launch(ctx, 0, granule, a, lr.list, s, 4);
+    st = spmm_long_launch(ctx, 0, a, lr.list, s, 4);
     if (st != AS_OK) cudaMemsetAsync(ctx->d_long, 0, 3 * sizeof(unsigned), s);
     return st;
 }
