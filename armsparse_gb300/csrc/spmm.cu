@@ -492,26 +492,65 @@ as_status spmm_launch(as_ctx *ctx, int dtype, int variant, const SpmmArgs &a, cu
     return st;
 }
 
-// The SpMM with the SDDMM fused in (spmm_nnz.cu): nnz-split variants only, one column tile.
-// Library choice: the narrowest full-warp tile that covers N (chunks of 1024 entries, four
-// entries per load batch -- the variants the autotuner picks for the power-law GCN layers).
+// Library choice for the fused pass, by entries and width, from sweeps on GB300 (graphs of 60k,
+// 574k, 15M and 35.8M entries, widths 8 to 256): the chunk is as long as leaves enough chunks to
+// fill the chip (a chunk is walked in order: 1024 entries take 0.2-0.3 ms by themselves, 128
+// about 50 us and 32 about 30 us; at 60k entries and width 48 in bf16 344 us with 1024, 30 with
+// 32; at 574k 315 with 1024, 62 with 128), and on a large graph narrow rows of B take the kernels
+// that bring several entries per load (35.8M entries, width 48, bf16: 2.55 ms with one entry per
+// warp step, 1.66 with two). Each class lists the narrowest tile first; a layout that none of a class
+// serves takes the 1024-entry kernels with 4- and 16-byte vectors, and one that those do not serve
+// is refused.
+struct FusedPick {
+    int kind, vb, group, cpl, chunk, steps;
+};
+static int fused_default(int dtype, const SpmmArgs &a, const SddmmFuse &f) {
+    const int esz = dtype == 0 ? 4 : 2;
+    const Variant *t = dtype == 0 ? kF32 : kBF16;
+    const int n = spmm_variant_count(dtype);
+    auto find = [&](const FusedPick &p) {
+        const int e = p.vb / esz;
+        if (e < 1 || e * p.group * p.cpl < a.N) return 0;
+        if (f.ldf % e || reinterpret_cast<uintptr_t>(f.F) % (e * esz)) return 0;
+        if (a.C16 && !(a.ldc % e == 0 && aligned(a.C16, 2 * e > 16 ? 16 : 2 * e))) return 0;
+        for (int i = 0; i < n; ++i)
+            if (t[i].kind == p.kind && t[i].vb == p.vb && t[i].group == p.group &&
+                t[i].cpl == p.cpl && t[i].unroll == p.chunk && (p.kind == 3 || t[i].steps == p.steps) &&
+                spmm_variant_supported(dtype, i + 1, a.N, a.ldb, a.ldc, a.B, a.C))
+                return i + 1;
+        return 0;
+    };
+    static const FusedPick large[] = {{3, 8, 8, 1, 1024, 4}, {3, 8, 16, 1, 1024, 4},
+                                      {2, 16, 16, 1, 256, 8}, {2, 16, 32, 1, 256, 8},
+                                      {2, 16, 32, 2, 256, 8}};
+    static const FusedPick medium[] = {{2, 4, 32, 1, 128, 4}, {2, 16, 16, 1, 128, 4},
+                                       {2, 16, 32, 1, 128, 4}, {2, 16, 32, 2, 128, 4}};
+    static const FusedPick small[] = {{2, 4, 32, 1, 32, 4}, {2, 4, 32, 2, 32, 4},
+                                      {2, 4, 32, 2, 128, 4}, {2, 16, 32, 1, 128, 4},
+                                      {2, 16, 32, 2, 128, 4}};
+    static const FusedPick any[] = {{2, 4, 32, 1, 1024, 4}, {2, 16, 32, 1, 1024, 4},
+                                    {2, 16, 32, 2, 1024, 4}};
+    auto first = [&](const FusedPick *p, int m) {
+        for (int i = 0; i < m; ++i)
+            if (const int v = find(p[i])) return v;
+        return 0;
+    };
+    const int fallback = first(any, 3);
+    if (fallback == 0) return 0;  // layouts that the fused pass does not serve
+    const int v = a.nnz >= 5000000 ? first(large, 5)
+                  : a.nnz >= 300000 ? first(medium, 4) : first(small, 5);
+    return v ? v : fallback;
+}
+
+// The SpMM with the SDDMM fused in (spmm_nnz.cu): nnz-split and multi-entry variants, one column
+// tile that covers N; variant 0 is the library's choice.
 as_status spmm_sddmm_launch(as_ctx *ctx, int dtype, int variant, const SpmmArgs &a,
                             const SddmmFuse &f, cudaStream_t s) {
     const int esz = dtype == 0 ? 4 : 2;
     const Variant *t = dtype == 0 ? kF32 : kBF16;
-    const int n = spmm_variant_count(dtype);
     auto tile = [&](const Variant &v) { return (v.vb / esz) * v.group * v.cpl; };
     if (variant == 0) {
-        const int picks[][3] = {{4, 32, 1}, {16, 32, 1}, {16, 32, 2}};  // vb, group, cpl
-        for (const auto &pk : picks) {
-            for (int i = 0; i < n && variant == 0; ++i)
-                if (t[i].kind == 2 && t[i].vb == pk[0] && t[i].group == pk[1] &&
-                    t[i].cpl == pk[2] && t[i].unroll == 1024 && t[i].steps == 4 &&
-                    tile(t[i]) >= a.N &&
-                    spmm_variant_supported(dtype, i + 1, a.N, a.ldb, a.ldc, a.B, a.C))
-                    variant = i + 1;
-            if (variant) break;
-        }
+        variant = fused_default(dtype, a, f);
         if (variant == 0)
             return fail(AS_ERR_UNSUPPORTED, "spmm+sddmm: no variant covers this N and layout");
     }

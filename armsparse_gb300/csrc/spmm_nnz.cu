@@ -2,11 +2,18 @@
 // skewed (power-law graphs), where one long row would serialise a row-per-group kernel.
 //
 // Pass 1 (spmm_nnzsplit): the entries are cut into chunks of CH consecutive entries; a group
-//   of GROUP lanes takes one chunk and one column tile, walks the chunk's row segments in CSR
-//   order and accumulates each segment with fmaf like the row-split kernels. A row that lies
-//   entirely inside the chunk is written to C directly (bit-identical to rowBaseSpmm3,
-//   SDMM.cpp:90-114). A row that crosses a chunk boundary leaves its segment's partial sum in
-//   a carry slot: slot 0 when the segment starts the chunk, slot 1 otherwise.
+//   of GROUP lanes takes one chunk and one column tile, and walks its entries in CSR order in
+//   steps of U, whatever rows they belong to: a batch of GROUP entries (one per lane), the ends
+//   of the next GROUP rows (one per lane) and from them a mask of the batch's row-ending
+//   entries are at hand before the batch starts, so the U rows of B of a step are loaded
+//   together across row ends, and the next batch's entries and row ends are loaded meanwhile.
+//   (Row by row, each row cost its pointer's, its entries' and its last 1-3 entries' memory
+//   latencies in turn: 57,442 rows of mean 10 at width 48 took 64 us and take 44; 1M rows, 15M
+//   entries, fp32 width 128: 1.04 and 0.92 ms.) Each row's segment is accumulated with fmaf like
+//   the row-split kernels. A row that lies entirely inside the chunk is written to C directly
+//   (bit-identical to rowBaseSpmm3, SDMM.cpp:90-114). A row that crosses a chunk boundary leaves
+//   its segment's partial sum in a carry slot: slot 0 when the segment starts the chunk, slot 1
+//   otherwise.
 // Pass 2 (spmm_nnz_fixup): for every row that ends inside chunk c after starting in an earlier
 //   chunk, chunk c's warp (a whole CTA for a long span) adds that row's partial sums (in chunk
 //   order when the row spans at most 8 chunks, else runs of chunks and then the runs in order;
@@ -23,6 +30,8 @@
 // entries the butterflies of all U run interleaved (each lane hands half of its values to its
 // partner at the first log2(U) steps), which pairs the same lanes in the same order, so each
 // dot product is the single-entry butterfly's bit for bit. One column tile only (TILE >= N).
+#include <limits.h>
+
 #include "common.cuh"
 #include "internal.h"
 #include "spmm_vec.cuh"
@@ -32,16 +41,38 @@ namespace {
 
 constexpr int kThreads = 256;
 
-__device__ __forceinline__ int find_row(const int *__restrict__ rowptr, int M, int e) {
-    int lo = 0, hi = M;  // largest r with rowptr[r] <= e
+// The row that holds entry e (largest r with rowptr[r] <= e), searched by a group of GROUP lanes:
+// each step probes GROUP points at once, so 2^21 rows take five dependent loads with 32 lanes,
+// not 21. Always in [0, M), whatever rowptr holds.
+template <int GROUP>
+__device__ __forceinline__ int find_row(const int *__restrict__ rowptr, int M, int e, int g,
+                                        unsigned gmask) {
+    long lo = 0, hi = M;
     while (hi - lo > 1) {
-        const int mid = (lo + hi) >> 1;
-        if (__ldg(rowptr + mid) <= e)
-            lo = mid;
-        else
-            hi = mid;
+        const long width = hi - lo;
+        const long probe = lo + width * (g + 1) / (GROUP + 1);
+        const int c = __popc(__ballot_sync(gmask, __ldg(rowptr + probe) <= e) & gmask);
+        const long nlo = c > 0 ? lo + width * c / (GROUP + 1) : lo;
+        const long nhi = c < GROUP ? lo + width * (c + 1) / (GROUP + 1) : hi;
+        lo = nlo;
+        hi = nhi;
     }
-    return lo;
+    return static_cast<int>(lo);
+}
+
+// A row segment's E sums at p, in whole vectors where the caller found them aligned.
+template <int E>
+__device__ __forceinline__ void store_f32(float *p, const float *v, bool vec) {
+    if constexpr (E % 4 == 0) {
+        if (vec) {
+#pragma unroll
+            for (int i = 0; i < E; i += 4)
+                *reinterpret_cast<float4 *>(p + i) = make_float4(v[i], v[i + 1], v[i + 2], v[i + 3]);
+            return;
+        }
+    }
+#pragma unroll
+    for (int i = 0; i < E; ++i) p[i] = v[i];
 }
 
 // Sum of each of the U values d[0..U) over the GROUP lanes of a group (U <= GROUP, both powers
@@ -93,17 +124,40 @@ __device__ __forceinline__ void write_dots(float (&d)[U], const int (&kk)[U], un
     if (g % SUB == 0 && ((ok >> u) & 1u)) store_dot(e0 + u, sum, nnz, perm, dA, status);
 }
 
+// kk * ldb_bytes on top of p: one wide multiply-add for rows of B under 4 GB, two
+// more instructions past that.
+__device__ __forceinline__ const char *row_at(const char *p, int kk, unsigned ldb_lo, unsigned ldb_hi) {
+    unsigned long long a;
+    asm("mad.wide.u32 %0, %1, %2, %3;" : "=l"(a) : "r"(kk), "r"(ldb_lo),
+        "l"(reinterpret_cast<unsigned long long>(p)));
+    if (ldb_hi) a += static_cast<unsigned long long>(static_cast<unsigned>(kk) * ldb_hi) << 32;
+    return reinterpret_cast<const char *>(a);
+}
+
+// A value as it travels between lanes, and as the step takes it.
+__device__ __forceinline__ float lane_val(float v) { return v; }
+__device__ __forceinline__ unsigned lane_val(uint16_t v) { return v; }
+
+// CTAs per SM to leave registers for: the gathers live on warps in flight, so four (64
+// registers) wherever a step's loads and the running sums fit, else two. (Width 256 in bf16 on
+// 35.8M entries: 2.14 ms with 64 registers, 2.54 with 76; fused 3.5 ms with 64 and a few
+// spilled, 5.4 with 100.)
+template <int VB, int CPL, int U, int E>
+constexpr int ctas_per_sm() { return U * CPL * VB / 4 + CPL * E <= 24 ? 4 : 2; }
+
 template <typename T, int VB, int GROUP, int CPL, int U, bool FUSE>
-__global__ void __launch_bounds__(kThreads)
+__global__ void __launch_bounds__(kThreads, ctas_per_sm<VB, CPL, U, Vec<T, VB>::E>())
 spmm_nnzsplit(int M, int K, int N, int nnz, int CH, const int *__restrict__ rowptr,
               const int *__restrict__ colind, const T *__restrict__ val,
               const T *__restrict__ B, long ldb, float *__restrict__ C, long ldc, float beta,
               float *__restrict__ carry, int *__restrict__ fix, unsigned *status,
               const T *__restrict__ F, long ldf, const int *__restrict__ perm,
-              float *__restrict__ dA, uint16_t *__restrict__ C16, bool relu) {
+              float *__restrict__ dA, uint16_t *__restrict__ C16, bool relu, bool c_vec,
+              bool carry_vec) {
     using V = Vec<T, VB>;
     constexpr int E = V::E;
     constexpr int TILE = GROUP * E * CPL;
+    static_assert(GROUP % U == 0, "a batch is whole steps");
     const int lane = threadIdx.x & 31;
     const int g = threadIdx.x % GROUP;
     const unsigned gmask =
@@ -112,174 +166,216 @@ spmm_nnzsplit(int M, int K, int N, int nnz, int CH, const int *__restrict__ rowp
     const long e0l = chunk * CH;
     if (e0l >= nnz) return;
     const int e0 = static_cast<int>(e0l);
-    const int e1 = static_cast<int>(e0l + CH < nnz ? e0l + CH : nnz);
+    // entries past the last row's end (a row pointer that stops short of nnz) belong to no row
+    const int e1 = static_cast<int>(
+        min(min(e0l + CH, static_cast<long>(nnz)), static_cast<long>(__ldg(rowptr + M))));
     const int tile0 = blockIdx.y * TILE;
-    int r = find_row(rowptr, M, e0);
-    int e = e0;
+    auto count = [&](bool p) { return __popc(__ballot_sync(gmask, p) & gmask); };
+    const char *bcol[CPL];  // this lane's columns of row 0 of B (column 0 for a lane past N)
+#pragma unroll
+    for (int j = 0; j < CPL; ++j) {
+        const int cc = tile0 + (j * GROUP + g) * E;
+        bcol[j] = reinterpret_cast<const char *>(B + (cc < N ? cc : 0));
+    }
+    const unsigned long long ldb_bytes = static_cast<unsigned long long>(ldb) * sizeof(T);
+    const unsigned ldb_lo = static_cast<unsigned>(ldb_bytes);
+    const unsigned ldb_hi = static_cast<unsigned>(ldb_bytes >> 32);
+
     int fix_row = -1;  // the row that started in an earlier chunk and ends in this one
-    while (e < e1 && r < M) {
-        const int rs = __ldg(rowptr + r), re = __ldg(rowptr + r + 1);
-        if (re <= e || rs > e) {  // empty row before e, or malformed pointers
-            if (rs > e || re < rs) {
-                flag(status, kFlagBadRowptr);
-                break;
-            }
-            ++r;
-            continue;
+    int r0 = e0 < e1 ? find_row<GROUP>(rowptr, M, e0, g, gmask) : 0;
+    const int rs0 = __ldg(rowptr + r0);
+    // the window of row ends: rows r, r + 1, ... (one per lane)
+    auto ends = [&](int r) {
+        const long i = static_cast<long>(r) + 1 + g;
+        return i <= M ? __ldg(rowptr + i) : INT_MAX;
+    };
+    // a window that may be used: never falling, its first past entry e
+    auto sound = [&](int w, int e) {
+        const int below = __shfl_up_sync(gmask, w, 1, GROUP);
+        return count(g > 0 ? w < below : w <= e) == 0;
+    };
+    using Val = decltype(lane_val(T()));
+    auto load_entry = [&](int e, int &k, Val &v) {
+        k = -1;
+        v = 0;
+        if (e < e1) {
+            k = ld_stream(colind + e);
+            v = lane_val(ld_stream(val + e));
         }
-        const int se = re < e1 ? re : e1;
-        const bool split = rs < e0 || re > e1;
-        if (rs < e0 && re <= e1) fix_row = r;
-        typename V::Raw fr[CPL];  // FUSE: this row's slices of F
-        if constexpr (FUSE) {
+    };
+    int re = ends(r0), k, base = e0;
+    Val v;
+    load_entry(base + g, k, v);
+    bool good = e0 < e1 && rs0 >= 0 && rs0 <= e0 && sound(re, e0);
+    if (e0 < e1 && !good) flag(status, kFlagBadRowptr);
+    int row = r0;                      // the row that the running sums belong to
+    int seg = e0;                      // its first entry in this chunk
+    const bool head_split = rs0 < e0;  // the chunk's first row started in an earlier chunk
+    float acc[CPL][E];
+    auto start_row = [&]() {
+#pragma unroll
+        for (int j = 0; j < CPL; ++j)
+#pragma unroll
+            for (int i = 0; i < E; ++i) acc[j][i] = 0.0f;
+        if (beta != 0.0f && row < M && __ldg(rowptr + row + 1) <= e1 && !(head_split && seg == e0)) {
 #pragma unroll
             for (int j = 0; j < CPL; ++j) {
                 const int cc = tile0 + (j * GROUP + g) * E;
-                fr[j] = V::raw(F + static_cast<long>(r) * ldf + (cc < N ? cc : 0));
+#pragma unroll
+                for (int i = 0; i < E; ++i)
+                    if (cc < N) acc[j][i] = beta * C[row * ldc + cc + i];
             }
         }
-        float acc[CPL][E];
-#pragma unroll
-        for (int j = 0; j < CPL; ++j) {
-            const int cc = tile0 + (j * GROUP + g) * E;
-#pragma unroll
-            for (int i = 0; i < E; ++i)
-                acc[j][i] = (!split && beta != 0.0f && cc < N) ? beta * C[r * ldc + cc + i] : 0.0f;
-        }
-        for (int base = e; base < se; base += GROUP) {
-            const int ee = base + g;
-            int k = -1;
-            float v = 0.0f;
-            if (ee < se) {
-                k = ld_stream(colind + ee);
-                v = to_f32(ld_stream(val + ee));
-                if (static_cast<unsigned>(k) >= static_cast<unsigned>(K)) {
-                    flag(status, kFlagBadColind);
-                    k = -1;
-                }
-            }
-            const int cnt = min(GROUP, se - base);
-            int t = 0;
-            // U entries per step, loads before FMAs (as in the row-split kernels: fp32 with
-            // per-load predicates, bf16 packed until the mixed-precision FMA)
-            for (; t + U <= cnt; t += U) {
-                int kk[U];
-                float vv[U];
-#pragma unroll
-                for (int u = 0; u < U; ++u) {
-                    kk[u] = __shfl_sync(gmask, k, t + u, GROUP);
-                    vv[u] = __shfl_sync(gmask, v, t + u, GROUP);
-                }
-                if constexpr (sizeof(T) == 4) {
-                    float b[U][CPL][E];
-#pragma unroll
-                    for (int u = 0; u < U; ++u) {
-                        const T *brow = B + static_cast<long>(kk[u] < 0 ? 0 : kk[u]) * ldb;
-#pragma unroll
-                        for (int j = 0; j < CPL; ++j) {
-                            const int cc = tile0 + (j * GROUP + g) * E;
-                            if (cc < N && kk[u] >= 0) {
-                                V::load(brow + cc, b[u][j]);
-                            } else {
-#pragma unroll
-                                for (int i = 0; i < E; ++i) b[u][j][i] = 0.0f;
-                            }
-                        }
-                    }
-#pragma unroll
-                    for (int u = 0; u < U; ++u)
-                        if (kk[u] >= 0)
-#pragma unroll
-                            for (int j = 0; j < CPL; ++j) fma_vec_f32<E>(b[u][j], vv[u], acc[j]);
-                    if constexpr (FUSE) {
-                        float d[U];
-#pragma unroll
-                        for (int u = 0; u < U; ++u) {
-                            d[u] = 0.0f;
-#pragma unroll
-                            for (int j = 0; j < CPL; ++j)
-                                if (tile0 + (j * GROUP + g) * E < N)
-#pragma unroll
-                                    for (int i = 0; i < E; ++i)
-                                        d[u] = fmaf(b[u][j][i], V::at(fr[j], i), d[u]);
-                        }
-                        write_dots<U, GROUP>(d, kk, gmask, g, base + t, nnz, perm, dA, status);
-                    }
-                } else {
-                    typename V::Raw b[U][CPL];
-#pragma unroll
-                    for (int u = 0; u < U; ++u) {
-                        const T *brow = B + static_cast<long>(kk[u] < 0 ? 0 : kk[u]) * ldb;
-#pragma unroll
-                        for (int j = 0; j < CPL; ++j) {
-                            const int cc = tile0 + (j * GROUP + g) * E;
-                            b[u][j] = V::raw(brow + (cc < N ? cc : 0));
-                        }
-                    }
-#pragma unroll
-                    for (int u = 0; u < U; ++u) {
-                        if (kk[u] < 0) continue;
-                        const unsigned short vu = static_cast<unsigned short>(__float_as_uint(vv[u]) >> 16);
-#pragma unroll
-                        for (int j = 0; j < CPL; ++j) V::fma(b[u][j], vu, acc[j]);
-                    }
-                    if constexpr (FUSE) {
-                        float d[U];
-#pragma unroll
-                        for (int u = 0; u < U; ++u) {
-                            d[u] = 0.0f;
-#pragma unroll
-                            for (int j = 0; j < CPL; ++j)
-                                if (tile0 + (j * GROUP + g) * E < N) V::dot(b[u][j], fr[j], d[u]);
-                        }
-                        write_dots<U, GROUP>(d, kk, gmask, g, base + t, nnz, perm, dA, status);
-                    }
-                }
-            }
-            for (; t < cnt; ++t) {
-                const int kk = __shfl_sync(gmask, k, t, GROUP);
-                const float vv = __shfl_sync(gmask, v, t, GROUP);
-                if (kk < 0) continue;
-                float d = 0.0f;
-#pragma unroll
-                for (int j = 0; j < CPL; ++j) {
-                    const int cc = tile0 + (j * GROUP + g) * E;
-                    if (cc < N) {
-                        float b[E];
-                        V::load(B + static_cast<long>(kk) * ldb + cc, b);
-#pragma unroll
-                        for (int i = 0; i < E; ++i) acc[j][i] = fmaf(b[i], vv, acc[j][i]);
-                        if constexpr (FUSE) {
-#pragma unroll
-                            for (int i = 0; i < E; ++i) d = fmaf(b[i], V::at(fr[j], i), d);
-                        }
-                    }
-                }
-                if constexpr (FUSE) {
-#pragma unroll
-                    for (int off = GROUP / 2; off >= 1; off >>= 1)
-                        d += __shfl_xor_sync(gmask, d, off, GROUP);
-                    if (g == 0) store_dot(base + t, d, nnz, perm, dA, status);
-                }
-            }
-        }
-        float *dst = split ? carry + (2 * chunk + (e == e0 ? 0 : 1)) * static_cast<long>(N)
-                           : C + r * ldc;
+    };
+    // the running sums to C, or (a row that goes on in another chunk) to a carry slot
+    auto store_row = [&](bool split) {
+        float *dst = split ? carry + (2 * chunk + (seg == e0 ? 0 : 1)) * static_cast<long>(N)
+                           : C + row * ldc;
+        const bool vec = split ? carry_vec : c_vec;
 #pragma unroll
         for (int j = 0; j < CPL; ++j) {
             const int cc = tile0 + (j * GROUP + g) * E;
             if (cc < N) {
-                if (!split && C16) {
-                    store_bf16<E>(C16 + r * ldc + cc, acc[j], relu);
-                } else {
-#pragma unroll
-                    for (int i = 0; i < E; ++i) dst[cc + i] = acc[j][i];
-                }
+                if (!split && C16)
+                    store_bf16<E>(C16 + row * ldc + cc, acc[j], relu);
+                else
+                    store_f32<E>(dst + cc, acc[j], vec);
             }
         }
-        e = se;
-        ++r;
+    };
+    start_row();
+    // FUSE: the slices of F of the running row
+    typename V::Raw fr[CPL];
+    auto start_f = [&]() {
+        if (row >= M) return;
+#pragma unroll
+        for (int j = 0; j < CPL; ++j) {
+            const int cc = tile0 + (j * GROUP + g) * E;
+            fr[j] = V::raw(F + static_cast<long>(row) * ldf + (cc < N ? cc : 0));
+        }
+    };
+    if constexpr (FUSE) start_f();
+
+    while (base < e1 && good) {
+        // This batch: entries base .. base + cnt - 1, cut where the window of row ends stops
+        // short of it (runs of empty rows).
+        const int last = __shfl_sync(gmask, re, GROUP - 1, GROUP);
+        const int cnt = min(min(GROUP, e1 - base), last - base);
+        const int next = base + cnt;
+        // bit i: entry base + i is its row's last
+        unsigned endm = re > base && re <= next ? 1u << (re - base - 1) : 0u;
+#pragma unroll
+        for (int off = GROUP / 2; off >= 1; off >>= 1)
+            endm |= __shfl_xor_sync(gmask, endm, off, GROUP);
+        // the next batch's entries and window, in flight meanwhile
+        int kn, rn = r0 + count(re <= next), ren = ends(rn);
+        Val vn;
+        load_entry(next + g, kn, vn);
+        if (g >= cnt) {
+            k = -1;
+        } else if (static_cast<unsigned>(k) >= static_cast<unsigned>(K)) {
+            flag(status, kFlagBadColind);
+            k = -1;
+        }
+        const bool clean = count(k >= 0) == GROUP;
+#pragma unroll 1
+        for (int t = 0; t < cnt; t += U) {
+            int kk[U];
+            Val vv[U];
+#pragma unroll
+            for (int u = 0; u < U; ++u) {
+                kk[u] = __shfl_sync(gmask, k, t + u, GROUP);
+                vv[u] = __shfl_sync(gmask, v, t + u, GROUP);
+            }
+            const unsigned em = endm >> t & ((1u << U) - 1u);
+            // U entries' rows of B before any is used (a skipped entry reads row 0)
+            typename V::Raw b[U][CPL];
+#pragma unroll
+            for (int u = 0; u < U; ++u)
+#pragma unroll
+                for (int j = 0; j < CPL; ++j)
+                    b[u][j] = V::raw(reinterpret_cast<const T *>(
+                        row_at(bcol[j], max(kk[u], 0), ldb_lo, ldb_hi)));
+            float d[U];
+            auto apply = [&](int u) {
+                d[u] = 0.0f;
+#pragma unroll
+                for (int j = 0; j < CPL; ++j) {
+                    const bool in = tile0 + (j * GROUP + g) * E < N;
+                    if constexpr (sizeof(T) == 4) {
+                        float bf[E];
+#pragma unroll
+                        for (int i = 0; i < E; ++i) bf[i] = V::at(b[u][j], i);
+                        fma_vec_f32<E>(bf, vv[u], acc[j]);
+                        if constexpr (FUSE) {
+                            float s = d[u];
+#pragma unroll
+                            for (int i = 0; i < E; ++i) s = fmaf(bf[i], V::at(fr[j], i), s);
+                            if (in) d[u] = s;
+                        }
+                    } else {
+                        V::fma(b[u][j], static_cast<unsigned short>(vv[u]), acc[j]);
+                        if constexpr (FUSE) {
+                            float s = d[u];
+                            V::dot(b[u][j], fr[j], s);
+                            if (in) d[u] = s;
+                        }
+                    }
+                }
+            };
+            if (GROUP == 32 && clean && em == 0) {
+#pragma unroll
+                for (int u = 0; u < U; ++u) apply(u);
+            } else {
+#pragma unroll
+                for (int u = 0; u < U; ++u) {
+                    d[u] = 0.0f;
+                    if (kk[u] >= 0) apply(u);
+                    if (em >> u & 1u) {  // the row ends here
+                        const bool split = head_split && seg == e0;
+                        store_row(split);
+                        if (split) fix_row = row;
+                        seg = base + t + u + 1;
+                        row = r0 + count(re <= seg);
+                        start_row();
+                        if constexpr (FUSE) start_f();
+                    }
+                }
+            }
+            if constexpr (FUSE) write_dots<U, GROUP>(d, kk, gmask, g, base + t, nnz, perm, dA, status);
+        }
+        // on to the next batch; where the window's rows all ended, look for the next row that
+        // holds an entry
+        if (next < e1) {
+            if (rn == r0 + GROUP) {
+                int empty = count(ren <= next);
+                while (empty == GROUP) {
+                    rn += GROUP;
+                    ren = ends(rn);
+                    empty = count(ren <= next);
+                }
+                if (empty) {
+                    rn += empty;
+                    ren = ends(rn);
+                }
+            }
+            if (!sound(ren, next)) {
+                flag(status, kFlagBadRowptr);
+                good = false;
+            }
+            if (row != rn) {  // the row after a run of empty ones
+                row = rn;
+                start_row();
+                if constexpr (FUSE) start_f();
+            }
+        }
+        r0 = rn;
+        re = ren;
+        k = kn;
+        v = vn;
+        base = next;
     }
+    if (good && seg < e1 && row < M) store_row(true);  // the last row goes on in the next chunk
     if (blockIdx.y == 0 && g == 0) fix[chunk] = fix_row;
 }
 
@@ -330,7 +426,7 @@ spmm_nnzme(int M, int K, int N, int nnz, int CH, const int *__restrict__ rowptr,
     const int e1 = static_cast<int>(e0l + CH < nnz ? e0l + CH : nnz);
     const int cc = blockIdx.y * TILE + g * E;  // this lane's columns
     const bool col_ok = cc < N;
-    int r = find_row(rowptr, M, e0);
+    int r = find_row<32>(rowptr, M, e0, lane, 0xffffffffu);
     int e = e0;
     int fix_row = -1;
     while (e < e1 && r < M) {  // uniform across the warp
@@ -648,13 +744,15 @@ as_status launch(as_ctx *ctx, const SpmmArgs &a, int CH, const SddmmFuse *fu, cu
                 FUSE ? static_cast<const T *>(fu->F) : nullptr, FUSE ? fu->ldf : 0,
                 FUSE ? fu->perm : nullptr, FUSE ? fu->dA : nullptr, a.C16, a.relu);
         } else {
+            const bool c_vec = a.ldc % 4 == 0 && reinterpret_cast<uintptr_t>(a.C) % 16 == 0;
             dim3 g1(static_cast<unsigned>(ceil_div(nchunks, kThreads / G)),
                     static_cast<unsigned>(ceil_div(a.N, TILE)));
             spmm_nnzsplit<T, VB, G, CPL, U, FUSE><<<g1, kThreads, 0, s>>>(
                 a.M, a.K, a.N, a.nnz, CH, a.rowptr, a.colind, static_cast<const T *>(a.val),
                 static_cast<const T *>(a.B), a.ldb, a.C, a.ldc, a.beta, carry, fix, a.status,
                 FUSE ? static_cast<const T *>(fu->F) : nullptr, FUSE ? fu->ldf : 0,
-                FUSE ? fu->perm : nullptr, FUSE ? fu->dA : nullptr, a.C16, a.relu);
+                FUSE ? fu->perm : nullptr, FUSE ? fu->dA : nullptr, a.C16, a.relu, c_vec,
+                a.N % 4 == 0);
         }
         dim3 g2(static_cast<unsigned>(ceil_div(nchunks, kFixChunks)));
         if (a.N % 4 == 0)  // carry rows are 16-byte aligned: whole-vector loads
@@ -674,9 +772,8 @@ as_status launch(as_ctx *ctx, const SpmmArgs &a, int CH, const SddmmFuse *fu, cu
 template <typename T, int VB, int G, int CPL>
 as_status launch_u(as_ctx *ctx, const SpmmArgs &a, int CH, int unroll, const SddmmFuse *fu,
                    cudaStream_t s) {
-    if (fu)
-        return unroll == 8 ? launch<T, VB, G, CPL, 8, true>(ctx, a, CH, fu, s)
-                           : launch<T, VB, G, CPL, 4, true>(ctx, a, CH, fu, s);
+    // fused: four entries per step whatever the variant (the sums do not depend on the step)
+    if (fu) return launch<T, VB, G, CPL, 4, true>(ctx, a, CH, fu, s);
     return unroll == 8 ? launch<T, VB, G, CPL, 8, false>(ctx, a, CH, fu, s)
                        : launch<T, VB, G, CPL, 4, false>(ctx, a, CH, fu, s);
 }

@@ -163,7 +163,9 @@ struct Vec<uint16_t, 2> {
 // (p aligned to min(2E, 16) bytes): the bf16 form of an fp32 output row segment. relu: negative
 // values are stored as 0 first (the epilogue of a layer followed by a ReLU).
 __device__ __forceinline__ unsigned pack_bf16x2(float lo, float hi) {
-    return static_cast<unsigned>(f32_to_bf16(lo)) | (static_cast<unsigned>(f32_to_bf16(hi)) << 16);
+    unsigned w;
+    asm("cvt.rn.bf16x2.f32 %0, %1, %2;" : "=r"(w) : "f"(hi), "f"(lo));
+    return w;
 }
 template <int E>
 __device__ __forceinline__ void store_bf16(uint16_t *p, const float *vin, bool relu = false) {
