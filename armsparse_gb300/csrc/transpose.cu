@@ -5,18 +5,29 @@
 // exactly the canonical CSC that scipy's tocsc() builds on the reference's GCN path
 // (gcn/pytorch-custom/gcn_custom.py:52), and the order the reference's counting transpose
 // (sparseTranspose.cpp:95-142) gives when its scatter runs in order. The sort is an LSD
-// radix sort over 8-bit digits of the column id, ceil(log2 N / 8) passes, each pass:
-//   1. tile histogram   -- each CTA counts the digits of its tile of kTile entries into
+// radix sort over digits of the column id, ceil(bits / 8) passes of equal width (20 bits: three
+// digits of 7), each pass:
+//   1. tile histogram   -- each CTA counts the digits of its tile of entries into
 //                          hist[digit * tiles + tile] (shared-memory atomics on counts:
 //                          the counts, unlike positions, do not depend on ordering);
 //   2. exclusive scan   -- over hist in (digit, tile) order, giving every (digit, tile) its
 //                          first output slot;
-//   3. stable scatter   -- each CTA re-reads its tile in rounds of 256 entries and ranks
-//                          every entry among equal digits that precede it (warp
-//                          __match_any_sync + per-warp counts + a running per-digit count),
-//                          parks the tile in shared memory sorted by digit, then writes
-//                          key, row and value out in that order, so each digit's entries
-//                          leave as one coalesced run.
+//   3. stable scatter   -- each warp of a CTA ranks the entries of its own consecutive part of
+//                          the tile among equal digits before them (a ballot per bit finds
+//                          the lanes of a digit, a warp-private count those before them), one scan over warps and digits turns
+//                          ranks into slots of the tile, the tile is parked in shared memory
+//                          sorted by digit, then key, row and value are written out in that
+//                          order, so each digit's entries leave as one coalesced run.
+// The first pass works out each entry's row from the row pointer as it goes (each row marks its
+// first entry in the tile, a running maximum gives the rest), so row ids are never written and
+// read just to be sorted.
+// What bounds a pass is its traffic (12 bytes read and written per entry) and how long the runs
+// are that leave a tile: 4096 entries and 128 digits give runs of 128 bytes. Measured on 16.8M
+// entries and 1M columns: a pass's scatter takes 110 us (2,048-entry tiles ranked in eight rounds
+// with a CTA barrier each: 166; ranks by __match_any_sync in place of the ballots: 150-169), the
+// rows 63 us more in the first pass (an expansion pass of its own: 79 us and its traffic), the
+// whole call 479 us (751 before). Matrices of few entries take tiles of 1024, which spread over
+// the chip (20,000 entries: 43 us, 68 before).
 // No position depends on timing, so the output is identical run to run. colptr comes
 // from the sorted keys (first slot of every column). All indices stay inside their
 // buffers for any input; malformed input sets the status word instead of faulting.
@@ -27,10 +38,13 @@ namespace as {
 namespace {
 
 constexpr int kThreads = 256;
-constexpr int kRounds = 8;
-constexpr int kTile = kThreads * kRounds;  // entries per tile
-constexpr int kBins = 256;
 constexpr int kWarps = kThreads / 32;
+constexpr int kSortThreads = 512;   // of a tile's CTA
+constexpr int kSortWarps = kSortThreads / 32;
+constexpr int kLargeItems = 8;      // entries per thread of a tile
+constexpr int kSmallItems = 2;
+constexpr int kLargeNnz = 300000;   // from here on large tiles (1M entries: 81 us, small ones 96)
+constexpr int kBins = 256;          // digits per pass at most
 
 // ---- exclusive scan of int32 (three phases, no cross-CTA waits) ---------------------------
 constexpr int kScanItems = 8;
@@ -77,225 +91,340 @@ scan_reduce(const int *__restrict__ in, long n, int *__restrict__ block_sums) {
     if (threadIdx.x == 0) block_sums[blockIdx.x] = total;
 }
 
-// Single CTA: exclusive scan of the block sums in place (any count, chunked).
-__global__ void __launch_bounds__(kThreads) scan_block_sums(int *sums, int nb) {
+// Each CTA adds up the sums of the CTAs before it, then scans its own chunk.
+__global__ void __launch_bounds__(kThreads)
+scan_downsweep(const int *__restrict__ in, long n, const int *__restrict__ block_sums,
+               int *__restrict__ out, bool vec) {
     __shared__ int sw[kWarps];
-    int carry = 0;
-    for (int base = 0; base < nb; base += kThreads) {
-        const int idx = base + threadIdx.x;
-        const int v = idx < nb ? sums[idx] : 0;
-        int total;
-        const int ex = block_exclusive_scan(v, sw, total);
-        if (idx < nb) sums[idx] = carry + ex;
-        carry += total;
+    const long base = static_cast<long>(blockIdx.x) * kScanChunk;
+    int before = 0;
+    for (int i = threadIdx.x; i < blockIdx.x; i += kThreads) before += block_sums[i];
+    int prefix;
+    block_exclusive_scan(before, sw, prefix);
+    // blocked layout: thread t owns items [t*kScanItems, (t+1)*kScanItems)
+    const long first = base + static_cast<long>(threadIdx.x) * kScanItems;
+    const bool whole = vec && first + kScanItems <= n;
+    int v[kScanItems];
+    int s = 0;
+    if (whole) {
+#pragma unroll
+        for (int i = 0; i < kScanItems; i += 4) {
+            const int4 q = *reinterpret_cast<const int4 *>(in + first + i);
+            v[i] = q.x; v[i + 1] = q.y; v[i + 2] = q.z; v[i + 3] = q.w;
+        }
+    } else {
+#pragma unroll
+        for (int i = 0; i < kScanItems; ++i) v[i] = first + i < n ? in[first + i] : 0;
+    }
+#pragma unroll
+    for (int i = 0; i < kScanItems; ++i) s += v[i];
+    int total;
+    int run = block_exclusive_scan(s, sw, total) + prefix;
+#pragma unroll
+    for (int i = 0; i < kScanItems; ++i) {
+        const int t = v[i];
+        v[i] = run;
+        run += t;
+    }
+    if (whole) {
+#pragma unroll
+        for (int i = 0; i < kScanItems; i += 4)
+            *reinterpret_cast<int4 *>(out + first + i) = make_int4(v[i], v[i + 1], v[i + 2], v[i + 3]);
+    } else {
+#pragma unroll
+        for (int i = 0; i < kScanItems; ++i)
+            if (first + i < n) out[first + i] = v[i];
     }
 }
 
-__global__ void __launch_bounds__(kThreads)
-scan_downsweep(const int *__restrict__ in, long n, const int *__restrict__ block_sums,
-               int *__restrict__ out) {
+// One CTA, n <= kScanChunk: the scan in place in one launch.
+__global__ void __launch_bounds__(kThreads) scan_one_block(int *data, long n) {
     __shared__ int sw[kWarps];
-    const long base = static_cast<long>(blockIdx.x) * kScanChunk;
-    // blocked layout: thread t owns items [t*kScanItems, (t+1)*kScanItems)
     int v[kScanItems];
     int s = 0;
 #pragma unroll
     for (int i = 0; i < kScanItems; ++i) {
-        const long idx = base + static_cast<long>(threadIdx.x) * kScanItems + i;
-        v[i] = idx < n ? in[idx] : 0;
+        const long idx = static_cast<long>(threadIdx.x) * kScanItems + i;
+        v[i] = idx < n ? data[idx] : 0;
         s += v[i];
     }
     int total;
-    int run = block_exclusive_scan(s, sw, total) + block_sums[blockIdx.x];
+    int run = block_exclusive_scan(s, sw, total);
 #pragma unroll
     for (int i = 0; i < kScanItems; ++i) {
-        const long idx = base + static_cast<long>(threadIdx.x) * kScanItems + i;
-        if (idx < n) out[idx] = run;
+        const long idx = static_cast<long>(threadIdx.x) * kScanItems + i;
+        if (idx < n) data[idx] = run;
         run += v[i];
     }
 }
 
 // ---- transpose kernels -----------------------------------------------------------------
-// rowidx[e] = row of entry e. Each thread takes kExpand consecutive entries: one binary
-// search over rowptr for its first entry, then it steps the row forward -- so one row with
-// millions of entries is spread over many threads. An entry that no well-formed row holds
-// (malformed pointers) is flagged and given row 0, so every row index written stays in [0, M)
-// and no slot keeps data from an earlier call.
-constexpr int kExpand = 8;
-__global__ void __launch_bounds__(kThreads)
-expand_rows(int M, int nnz, const int *__restrict__ rowptr, int *__restrict__ rowidx,
-            unsigned *status) {
-    const long e0 = (static_cast<long>(blockIdx.x) * kThreads + threadIdx.x) * kExpand;
-    if (e0 >= nnz) return;
-    int lo = 0, hi = M;  // largest r with rowptr[r] <= e0 (rowptr monotone for valid input)
-    while (hi - lo > 1) {
-        const int mid = (lo + hi) >> 1;
-        if (__ldg(rowptr + mid) <= e0)
-            lo = mid;
-        else
-            hi = mid;
+// Inclusive maximum over the CTA's threads before and with each (values >= 0).
+__device__ __forceinline__ int block_max_scan(int v, int *smem_warp) {
+    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+#pragma unroll
+    for (int o = 1; o < 32; o <<= 1) {
+        const int y = __shfl_up_sync(0xffffffffu, v, o);
+        if (lane >= o) v = max(v, y);
     }
-    int r = lo;
-    int rs = __ldg(rowptr + r), re = __ldg(rowptr + r + 1);
-    const long e1 = e0 + kExpand < nnz ? e0 + kExpand : nnz;
-    for (long e = e0; e < e1; ++e) {
-        while (e >= re && r + 1 < M) {  // advance to the row that holds e
-            ++r;
-            rs = re;
-            re = __ldg(rowptr + r + 1);
-        }
-        if (rs < 0 || re < rs || re > nnz || e < rs || e >= re) {
-            flag(status, kFlagBadRowptr);
-            rowidx[e] = 0;  // malformed pointers: an in-range row, never stale scratch
-            continue;
-        }
-        rowidx[e] = r;
-    }
-}
-
-__global__ void __launch_bounds__(kThreads)
-check_rowptr_ends(int M, int nnz, const int *__restrict__ rowptr, int *__restrict__ rowidx,
-                  unsigned *status) {
-    // rowptr[0] must be 0 and rowptr[M] == nnz; otherwise some rowidx slots would be stale:
-    // zero them so the sort reads defined data, and flag.
-    const int first = __ldg(rowptr), last = __ldg(rowptr + M);
-    if (first != 0 || last != nnz) {
-        if (blockIdx.x == 0 && threadIdx.x == 0) flag(status, kFlagBadRowptr);
-        for (long e = static_cast<long>(blockIdx.x) * kThreads + threadIdx.x; e < nnz;
-             e += static_cast<long>(gridDim.x) * kThreads)
-            rowidx[e] = 0;
-    }
-}
-
-__global__ void __launch_bounds__(kThreads)
-radix_histogram(const int *__restrict__ keys, int nnz, int shift, int tiles, int N,
-                int *__restrict__ hist, unsigned *status, int check_range) {
-    __shared__ int h[kBins];
-    h[threadIdx.x] = 0;
+    if (lane == 31) smem_warp[warp] = v;
     __syncthreads();
-    const long base = static_cast<long>(blockIdx.x) * kTile;
-    int kv[kRounds];  // all of this thread's keys are loaded before any is counted
+    for (int w = 0; w < warp; ++w) v = max(v, smem_warp[w]);
+    __syncthreads();
+    return v;
+}
+
+// Largest r in [0, M) with rowptr[r] <= e, by a whole warp (32 probes per step).
+__device__ __forceinline__ int warp_find_row(int M, const int *__restrict__ rowptr, long e) {
+    const int lane = threadIdx.x & 31;
+    long lo = 0, hi = M;
+    while (hi - lo > 1) {
+        const long width = hi - lo;
+        const long probe = lo + width * (lane + 1) / 33;
+        const int c = __popc(__ballot_sync(0xffffffffu, __ldg(rowptr + probe) <= e));
+        const long nlo = c > 0 ? lo + width * c / 33 : lo;
+        const long nhi = c < 32 ? lo + width * (c + 1) / 33 : hi;
+        lo = nlo;
+        hi = nhi;
+    }
+    return static_cast<int>(lo);
+}
+
+template <int ITEMS>
+__global__ void __launch_bounds__(kSortThreads)
+radix_histogram(const int *__restrict__ keys, int nnz, int shift, int bins, int tiles, int N,
+                int *__restrict__ hist, unsigned *status, int check_range, bool vec) {
+    __shared__ int h[kBins];
+    if (threadIdx.x < kBins) h[threadIdx.x] = 0;
+    __syncthreads();
+    const long base = static_cast<long>(blockIdx.x) * kSortThreads * ITEMS;
+    int kv[ITEMS];  // all of this thread's keys are loaded before any is counted
+    const long first = base + static_cast<long>(threadIdx.x) * ITEMS;
+    int n = ITEMS;
+    if (ITEMS % 4 == 0 && vec && base + kSortThreads * ITEMS <= nnz) {
 #pragma unroll
-    for (int i = 0; i < kRounds; ++i) {
-        const long idx = base + static_cast<long>(i) * kThreads + threadIdx.x;
-        kv[i] = idx < nnz ? keys[idx] : 0;
+        for (int i = 0; i + 3 < ITEMS; i += 4) {
+            const int4 q = *reinterpret_cast<const int4 *>(keys + first + i);
+            kv[i] = q.x; kv[i + 1] = q.y; kv[i + 2] = q.z; kv[i + 3] = q.w;
+        }
+    } else {
+        n = static_cast<int>(min(static_cast<long>(ITEMS), max(0L, nnz - first)));
+#pragma unroll
+        for (int i = 0; i < ITEMS; ++i) kv[i] = i < n ? keys[first + i] : 0;
     }
 #pragma unroll
-    for (int i = 0; i < kRounds; ++i) {
-        const long idx = base + static_cast<long>(i) * kThreads + threadIdx.x;
-        if (idx < nnz) {
+    for (int i = 0; i < ITEMS; ++i) {
+        if (i < n) {
             const int k = kv[i];
             if (check_range && static_cast<unsigned>(k) >= static_cast<unsigned>(N))
                 flag(status, kFlagBadColind);
-            atomicAdd(&h[(static_cast<unsigned>(k) >> shift) & (kBins - 1)], 1);
+            atomicAdd(&h[(static_cast<unsigned>(k) >> shift) & (bins - 1)], 1);
         }
     }
     __syncthreads();
-    hist[static_cast<long>(threadIdx.x) * tiles + blockIdx.x] = h[threadIdx.x];
+    if (threadIdx.x < bins)
+        hist[static_cast<long>(threadIdx.x) * tiles + blockIdx.x] = h[threadIdx.x];
 }
 
-__global__ void __launch_bounds__(kThreads)
+// rows null: the first pass, rows from rowptr (an entry that no well-formed row holds is flagged
+// and given row 0, as are all when the pointer does not run from 0 to nnz, so every row written
+// is in [0, M)). vals null: no payload, or with iota each entry's position.
+template <int ITEMS>
+__global__ void __launch_bounds__(kSortThreads, 2)
 radix_scatter(const int *__restrict__ keys, const int *__restrict__ rows,
-              const unsigned *__restrict__ vals, bool iota, int nnz, int shift, int tiles,
+              const unsigned *__restrict__ vals, bool iota, int nnz, int shift, int bins, int tiles,
               const int *__restrict__ offsets, int *__restrict__ okeys, int *__restrict__ orows,
-              unsigned *__restrict__ ovals) {
-    static_assert(kBins == kThreads, "one digit per thread");
-    __shared__ int run[kBins];            // running local slot per digit inside this tile
-    __shared__ int start[kBins];          // first local slot of each digit in this tile
-    __shared__ int goff[kBins];           // first global slot of each digit for this tile
-    __shared__ int wcnt[kWarps][kBins];   // per-warp counts of the current round
-    __shared__ int sw[kWarps];
-    __shared__ int sk[kTile];             // the tile, sorted by digit (stable)
-    __shared__ int sr[kTile];
-    __shared__ unsigned sv[kTile];  // the payload: value bits or entry index
-    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+              unsigned *__restrict__ ovals, int M, const int *__restrict__ rowptr,
+              unsigned *status) {
+    constexpr int kTile = kSortThreads * ITEMS;
+    __shared__ int start[kBins];               // first local slot of each digit in this tile
+    __shared__ int goff[kBins];                // its first global slot, less the local one
+    __shared__ unsigned short cnt[kSortWarps][kBins];  // per warp and digit: count, then first slot
+    __shared__ int sw[kSortWarps];
+    __shared__ int row_span[2];
+    extern __shared__ int parked[];            // the tile, sorted by digit (stable)
+    int *sk = parked, *sr = parked + kTile;
+    unsigned *sv = reinterpret_cast<unsigned *>(parked + 2 * kTile);  // value bits or position
+    const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
     const long base = static_cast<long>(blockIdx.x) * kTile;
     const int n_tile = static_cast<int>(nnz - base < kTile ? nnz - base : kTile);
-    {   // this tile's digit counts from the scanned (digit, tile) offsets; local starts
-        const long idx = static_cast<long>(threadIdx.x) * tiles + blockIdx.x;
-        const int off = offsets[idx];
-        const int nxt = idx + 1 < static_cast<long>(kBins) * tiles ? offsets[idx + 1] : nnz;
-        int total;
-        const int st = block_exclusive_scan(nxt - off, sw, total);
-        goff[threadIdx.x] = off;
-        start[threadIdx.x] = st;
-        run[threadIdx.x] = st;
-    }
-    const unsigned lt_mask = (1u << lane) - 1u;
-    int kr[kRounds], rr[kRounds];  // the thread's entries, loaded before the ranking rounds
-    unsigned vr[kRounds];
+    const int w0 = warp * (32 * ITEMS) + lane;  // this lane's first entry in the tile
+    int kr[ITEMS], rr[ITEMS];
+    unsigned vr[ITEMS];
 #pragma unroll
-    for (int i = 0; i < kRounds; ++i) {
-        const int li = i * kThreads + threadIdx.x;
+    for (int i = 0; i < ITEMS; ++i) {
+        const int li = w0 + 32 * i;
         kr[i] = 0;
         rr[i] = 0;
         vr[i] = 0u;
         if (li < n_tile) {
             kr[i] = keys[base + li];
-            rr[i] = rows[base + li];
+            if (rows) rr[i] = rows[base + li];
             if (vals)
                 vr[i] = vals[base + li];
             else if (iota)
                 vr[i] = static_cast<unsigned>(base + li);  // the entry's CSR position
         }
     }
-#pragma unroll
-    for (int i = 0; i < kRounds; ++i) {
-        const int li = i * kThreads + threadIdx.x;
-        const bool valid = li < n_tile;
-        const int k = kr[i], r = rr[i];
-        const unsigned v = vr[i];
-        const int d = valid ? static_cast<int>((static_cast<unsigned>(k) >> shift) & (kBins - 1))
-                            : kBins;  // invalid lanes get a digit of their own
-#pragma unroll
-        for (int w = 0; w < kWarps; ++w) wcnt[w][threadIdx.x] = 0;
+    for (int i = tid; i < kSortWarps * kBins; i += kSortThreads) (&cnt[0][0])[i] = 0;
+    if (!rows) {
+        // Rows of the tile's entries: each row marks its first entry of the tile (of rows that
+        // start at one entry the last is the one that holds it), and the running maximum over
+        // the tile is every entry's row.
+        const bool ends = __ldg(rowptr) == 0 && __ldg(rowptr + M) == nnz;
+        if (!ends && tid == 0 && blockIdx.x == 0) flag(status, kFlagBadRowptr);
+        if (warp < 2) {
+            const int r = warp_find_row(M, rowptr, warp == 0 ? base : base + n_tile - 1);
+            if (lane == 0) row_span[warp] = r;
+        }
+        for (int i = tid; i < kTile; i += kSortThreads) sr[i] = 0;
         __syncthreads();
-        const unsigned peers = __match_any_sync(0xffffffffu, d);
-        const int rank = __popc(peers & lt_mask);
-        if (valid && rank == 0) wcnt[warp][d] = __popc(peers);
+        const int ra = row_span[0], rb = row_span[1];
+        for (long r = static_cast<long>(ra) + tid; r <= rb; r += kSortThreads) {
+            const long at = static_cast<long>(__ldg(rowptr + r)) - base;
+            if (r == ra || (at > 0 && at < n_tile))
+                atomicMax(sr + (r == ra ? 0 : at), static_cast<int>(r));
+        }
         __syncthreads();
-        {   // per digit: exclusive prefix over warps, then advance the running count
-            const int dd = threadIdx.x;
-            int acc = run[dd];
+        int m = 0, mine[ITEMS];
 #pragma unroll
-            for (int w = 0; w < kWarps; ++w) {
-                const int c = wcnt[w][dd];
-                wcnt[w][dd] = acc;
+        for (int i = 0; i < ITEMS; ++i) {
+            m = max(m, sr[tid * ITEMS + i]);
+            mine[i] = m;
+        }
+        const int upto = block_max_scan(m, sw);
+        int prev = __shfl_up_sync(0xffffffffu, upto, 1);
+        if (lane == 0) sw[warp] = 0;
+        __syncthreads();
+        if (lane == 31 && warp + 1 < kSortWarps) sw[warp + 1] = upto;
+        __syncthreads();
+        if (lane == 0) prev = sw[warp];
+#pragma unroll
+        for (int i = 0; i < ITEMS; ++i) sr[tid * ITEMS + i] = max(mine[i], prev);
+        __syncthreads();
+#pragma unroll
+        for (int i = 0; i < ITEMS; ++i) {
+            const int li = w0 + 32 * i;
+            if (!ends || li >= n_tile) continue;
+            const int r = sr[li];
+            const long e = base + li;
+            const int rs = __ldg(rowptr + r), re = __ldg(rowptr + r + 1);
+            if (rs < 0 || re > nnz || e < rs || e >= re)
+                flag(status, kFlagBadRowptr);  // malformed pointers: row 0
+            else
+                rr[i] = r;
+        }
+    }
+    __syncthreads();
+    // ranks among equal digits of the warp's entries before each
+    const unsigned lt_mask = (1u << lane) - 1u;
+    unsigned short *mine = cnt[warp];
+    // lanes whose digit is this lane's: a ballot per bit
+    unsigned peers[ITEMS];
+#pragma unroll
+    for (int i = 0; i < ITEMS; ++i)
+        peers[i] = __ballot_sync(0xffffffffu, w0 + 32 * i < n_tile);
+    for (int bit = 1; bit < bins; bit <<= 1) {
+#pragma unroll
+        for (int i = 0; i < ITEMS; ++i) {
+            const bool one = (static_cast<unsigned>(kr[i]) >> shift) & bit;
+            const unsigned m = __ballot_sync(0xffffffffu, one);
+            peers[i] &= one ? m : ~m;
+        }
+    }
+    int rank[ITEMS];
+#pragma unroll
+    for (int i = 0; i < ITEMS; ++i) {
+        const bool valid = w0 + 32 * i < n_tile;
+        const int d = static_cast<int>((static_cast<unsigned>(kr[i]) >> shift) & (bins - 1));
+        const int lower = __popc(peers[i] & lt_mask);
+        const int before = valid ? mine[d] : 0;
+        __syncwarp();
+        if (valid && lower == 0) mine[d] = static_cast<unsigned short>(before + __popc(peers[i]));
+        __syncwarp();
+        rank[i] = before + lower;
+    }
+    __syncthreads();
+    {   // per digit: exclusive prefix over warps; then over digits
+        int acc = 0;
+        if (tid < bins) {
+#pragma unroll
+            for (int w = 0; w < kSortWarps; ++w) {
+                const int c = cnt[w][tid];
+                cnt[w][tid] = static_cast<unsigned short>(acc);
                 acc += c;
             }
-            run[dd] = acc;
         }
+        int v = acc;
+#pragma unroll
+        for (int o = 1; o < 32; o <<= 1) {
+            const int y = __shfl_up_sync(0xffffffffu, v, o);
+            if (lane >= o) v += y;
+        }
+        if (lane == 31) sw[warp] = v;
         __syncthreads();
-        if (valid) {
-            const int pos = wcnt[warp][d] + rank;
-            sk[pos] = k;
-            sr[pos] = r;
-            sv[pos] = v;
+        int st = v - acc;
+        for (int w = 0; w < warp; ++w) st += sw[w];
+        if (tid < bins) {
+            start[tid] = st;
+            goff[tid] = offsets[static_cast<long>(tid) * tiles + blockIdx.x] - st;
         }
-        __syncthreads();  // wcnt is cleared by the next round
     }
+    __syncthreads();
+#pragma unroll
+    for (int i = 0; i < ITEMS; ++i) {
+        if (w0 + 32 * i < n_tile) {
+            const int d = static_cast<int>((static_cast<unsigned>(kr[i]) >> shift) & (bins - 1));
+            const int pos = start[d] + mine[d] + rank[i];
+            sk[pos] = kr[i];
+            sr[pos] = rr[i];
+            sv[pos] = vr[i];
+        }
+    }
+    __syncthreads();
     // write out in local (digit-sorted) order: a digit's entries go to consecutive global
     // slots, so neighbouring threads write neighbouring addresses
-    for (int p = threadIdx.x; p < n_tile; p += kThreads) {
-        const int k = sk[p];
-        const int d = static_cast<int>((static_cast<unsigned>(k) >> shift) & (kBins - 1));
-        const int g = goff[d] + (p - start[d]);
-        okeys[g] = k;
-        orows[g] = sr[p];
-        if (ovals) ovals[g] = sv[p];
+#pragma unroll
+    for (int i = 0; i < ITEMS; ++i) {
+        const int p = tid + i * kSortThreads;
+        if (p < n_tile) {
+            const int k = sk[p];
+            const int g = goff[(static_cast<unsigned>(k) >> shift) & (bins - 1)] + p;
+            okeys[g] = k;
+            orows[g] = sr[p];
+            if (ovals) ovals[g] = sv[p];
+        }
     }
 }
 
-// colptr[c] = first slot whose key >= c, from the sorted keys.
+// colptr[c] = first slot whose key >= c, from the sorted keys (256-byte aligned scratch): eight
+// consecutive slots per thread.
+constexpr int kColSlots = 8;
 __global__ void __launch_bounds__(kThreads)
 colptr_from_keys(const int *__restrict__ skeys, int nnz, int N, int *__restrict__ colptr) {
-    const long p = static_cast<long>(blockIdx.x) * kThreads + threadIdx.x;
-    if (p > nnz) return;
-    long kprev = p == 0 ? -1 : skeys[p - 1];
-    long kcur = p == nnz ? N : skeys[p];
-    if (kprev < -1) kprev = -1;
-    if (kcur > N) kcur = N;
-    for (long c = kprev + 1; c <= kcur; ++c) colptr[c] = static_cast<int>(p);
+    const long p0 = (static_cast<long>(blockIdx.x) * kThreads + threadIdx.x) * kColSlots;
+    if (p0 > nnz) return;
+    int k[kColSlots];
+    if (p0 + kColSlots <= nnz) {
+#pragma unroll
+        for (int i = 0; i < kColSlots; i += 4) {
+            const int4 v = *reinterpret_cast<const int4 *>(skeys + p0 + i);
+            k[i] = v.x; k[i + 1] = v.y; k[i + 2] = v.z; k[i + 3] = v.w;
+        }
+    } else {
+#pragma unroll
+        for (int i = 0; i < kColSlots; ++i) k[i] = p0 + i < nnz ? skeys[p0 + i] : N;
+    }
+    // keys out of range were flagged: clamped to [-1, N] they move no column pointer out of place
+    int prev = p0 == 0 ? -1 : max(skeys[p0 - 1], -1);
+#pragma unroll
+    for (int i = 0; i < kColSlots; ++i) {
+        if (p0 + i > nnz) break;
+        const int p = static_cast<int>(p0) + i;
+        const int cur = p == nnz ? N : min(k[i], N);
+        for (int c = prev + 1; c <= cur && prev < N; ++c) colptr[c] = p;
+        prev = max(k[i], -1);
+    }
 }
 
 // ---- validation --------------------------------------------------------------------------
@@ -328,11 +457,17 @@ f32_to_bf16_kernel(long n, const float *__restrict__ src, uint16_t *__restrict__
 
 __global__ void zero_u32(unsigned *p) { *p = 0u; }
 
-int radix_passes(int N) {
-    int bits = 0;
+// Digits of an N-column matrix: as few passes as digits of at most 8 bits give, of equal width.
+struct Digits {
+    int passes, bits;
+};
+Digits radix_digits(int N) {
+    int bits = 1;
     while (bits < 31 && (1L << bits) < N) ++bits;
-    return bits <= 8 ? 1 : (bits + 7) / 8;
+    const int passes = (bits + 7) / 8;
+    return {passes, (bits + passes - 1) / passes};
 }
+int tile_entries(int nnz) { return kSortThreads * (nnz >= kLargeNnz ? kLargeItems : kSmallItems); }
 
 size_t align256(size_t b) { return (b + 255) & ~size_t(255); }
 
@@ -344,9 +479,9 @@ static as_status exclusive_scan(as_ctx *ctx, const int *in, int *out, long n, in
     const long nb = ceil_div(n, kScanChunk);
     if (nb == 0) return AS_OK;
     scan_reduce<<<static_cast<unsigned>(nb), kThreads, 0, s>>>(in, n, work);
-    scan_block_sums<<<1, kThreads, 0, s>>>(work, static_cast<int>(nb));
-    scan_downsweep<<<static_cast<unsigned>(nb), kThreads, 0, s>>>(in, n, work, out);
-    ctx->launches += 3;
+    const bool vec = (reinterpret_cast<uintptr_t>(in) | reinterpret_cast<uintptr_t>(out)) % 16 == 0;
+    scan_downsweep<<<static_cast<unsigned>(nb), kThreads, 0, s>>>(in, n, work, out, vec);
+    ctx->launches += 2;
     return check_cuda(cudaGetLastError(), "scan launch");
 }
 
@@ -357,17 +492,84 @@ as_status exclusive_scan_i32(as_ctx *ctx, const int *in, int *out, long n, cudaS
     return exclusive_scan(ctx, in, out, n, static_cast<int *>(w), s);
 }
 
+// Raw launches of the passes, shared by the two entry points (the caller reads the launch error).
+// Keys alternate between keysA and keysB. Rows and values of a non-last pass go to either the
+// scratch buffer or the caller's output (free until the last pass), chosen backwards from the
+// last pass so that no pass reads and writes the same buffer and the last pass reads scratch and
+// writes rowind / final_v. Returns the number of launches.
+struct SortBuffers {
+    int *keysA, *keysB, *rowsT;
+    unsigned *valsT;
+    int *hist, *sums;
+};
+static int sort_by_column(int M, int N, int nnz, const int *rowptr, const int *colind,
+                          const unsigned *vals, bool iota, int *colptr, int *rowind,
+                          unsigned *final_v, const SortBuffers &w, unsigned *status,
+                          cudaStream_t s) {
+    const Digits dg = radix_digits(N);
+    const int bins = 1 << dg.bits;
+    const bool large = nnz >= kLargeNnz;
+    const int tile = tile_entries(nnz);
+    const unsigned tiles = static_cast<unsigned>(ceil_div(nnz, tile));
+    const long hist_n = static_cast<long>(tiles) * bins;
+    const unsigned nb = static_cast<unsigned>(ceil_div(hist_n, kScanChunk));
+    const size_t smem = 3 * sizeof(int) * static_cast<size_t>(tile);
+    int launches = 0;
+    if (large)  // past the 48 KB that need no opt-in, with the static arrays
+        cudaFuncSetAttribute(radix_scatter<kLargeItems>, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                             static_cast<int>(smem));
+    const int *src_k = colind;
+    const int *src_r = nullptr;  // the first pass takes them from rowptr
+    const unsigned *src_v = vals;
+    for (int pass = 0; pass < dg.passes; ++pass) {
+        const bool last = pass == dg.passes - 1;
+        const bool to_scratch = ((dg.passes - 1 - pass) & 1) != 0;
+        int *dk = (pass & 1) ? w.keysB : w.keysA;
+        int *dr = (last || !to_scratch) ? rowind : w.rowsT;
+        unsigned *dv = final_v ? ((last || !to_scratch) ? final_v : w.valsT) : nullptr;
+        const int shift = dg.bits * pass;
+        const bool vec = reinterpret_cast<uintptr_t>(src_k) % 16 == 0;
+        if (large)
+            radix_histogram<kLargeItems><<<tiles, kSortThreads, 0, s>>>(
+                src_k, nnz, shift, bins, tiles, N, w.hist, status, pass == 0, vec);
+        else
+            radix_histogram<kSmallItems><<<tiles, kSortThreads, 0, s>>>(
+                src_k, nnz, shift, bins, tiles, N, w.hist, status, pass == 0, vec);
+        if (nb == 1) {
+            scan_one_block<<<1, kThreads, 0, s>>>(w.hist, hist_n);
+            launches += 1;
+        } else {
+            scan_reduce<<<nb, kThreads, 0, s>>>(w.hist, hist_n, w.sums);
+            scan_downsweep<<<nb, kThreads, 0, s>>>(w.hist, hist_n, w.sums, w.hist, true);
+            launches += 2;
+        }
+        if (large)
+            radix_scatter<kLargeItems><<<tiles, kSortThreads, smem, s>>>(
+                src_k, src_r, src_v, iota && pass == 0, nnz, shift, bins, tiles, w.hist, dk, dr, dv, M,
+                rowptr, status);
+        else
+            radix_scatter<kSmallItems><<<tiles, kSortThreads, smem, s>>>(
+                src_k, src_r, src_v, iota && pass == 0, nnz, shift, bins, tiles, w.hist, dk, dr, dv, M,
+                rowptr, status);
+        launches += 2;
+        src_k = dk;
+        src_r = dr;
+        src_v = dv;
+    }
+    colptr_from_keys<<<static_cast<unsigned>(ceil_div(static_cast<long>(nnz) + 1,
+                                                      kThreads * kColSlots)),
+                       kThreads, 0, s>>>(src_k, nnz, N, colptr);
+    return launches + 1;
+}
+
 size_t csr2csc_scratch_bytes(int nnz, int N, bool with_val) {
-    const long tiles = ceil_div(nnz, kTile);
-    const long hist = tiles * kBins;
+    const long hist = ceil_div(nnz, tile_entries(nnz)) << radix_digits(N).bits;
     size_t b = 0;
-    b += align256(sizeof(int) * static_cast<size_t>(nnz));        // rowidx
     b += 2 * align256(sizeof(int) * static_cast<size_t>(nnz));    // keys ping-pong
     b += align256(sizeof(int) * static_cast<size_t>(nnz));        // rows (intermediate)
     if (with_val) b += align256(sizeof(float) * static_cast<size_t>(nnz));
     b += align256(sizeof(int) * static_cast<size_t>(hist));       // histogram / offsets
     b += align256(sizeof(int) * static_cast<size_t>(ceil_div(hist, kScanChunk) + 1));
-    (void)N;
     return b;
 }
 
@@ -383,56 +585,21 @@ as_status csr2csc_launch(as_ctx *ctx, int M, int N, int nnz, const int *rowptr,
     if (N == 0) return fail(AS_ERR_INVALID_CSR, "csr2csc: nnz > 0 with zero columns");
     // the payload: the values' bits, or (perm given) each entry's CSR position
     const bool wv = val != nullptr || perm != nullptr;
-    unsigned *final_v = perm ? reinterpret_cast<unsigned *>(perm)
-                             : reinterpret_cast<unsigned *>(cscval);
-    const int tiles = static_cast<int>(ceil_div(nnz, kTile));
-    const long hist_n = static_cast<long>(tiles) * kBins;
+    unsigned *final_v = !wv ? nullptr : perm ? reinterpret_cast<unsigned *>(perm)
+                                             : reinterpret_cast<unsigned *>(cscval);
+    const long hist_n = ceil_div(nnz, tile_entries(nnz)) << radix_digits(N).bits;
     char *p = static_cast<char *>(work);
     auto take = [&](size_t bytes) { char *q = p; p += align256(bytes); return q; };
-    int *rowidx = reinterpret_cast<int *>(take(sizeof(int) * static_cast<size_t>(nnz)));
-    int *keysA = reinterpret_cast<int *>(take(sizeof(int) * static_cast<size_t>(nnz)));
-    int *keysB = reinterpret_cast<int *>(take(sizeof(int) * static_cast<size_t>(nnz)));
-    int *rowsT = reinterpret_cast<int *>(take(sizeof(int) * static_cast<size_t>(nnz)));
-    unsigned *valsT = wv ? reinterpret_cast<unsigned *>(take(sizeof(unsigned) * static_cast<size_t>(nnz))) : nullptr;
-    int *hist = reinterpret_cast<int *>(take(sizeof(int) * static_cast<size_t>(hist_n)));
-    int *sums = reinterpret_cast<int *>(take(sizeof(int) * static_cast<size_t>(ceil_div(hist_n, kScanChunk) + 1)));
-
-    const unsigned gw = static_cast<unsigned>(ceil_div(ceil_div(nnz, kExpand), kThreads));
-    expand_rows<<<gw, kThreads, 0, s>>>(M, nnz, rowptr, rowidx, ctx->d_status);
-    check_rowptr_ends<<<static_cast<unsigned>(ceil_div(nnz, kThreads) < 4096 ? ceil_div(nnz, kThreads) : 4096),
-                        kThreads, 0, s>>>(M, nnz, rowptr, rowidx, ctx->d_status);
-    ctx->launches += 2;
-
-    // Keys alternate between keysA and keysB. Rows and values of a non-last pass go to
-    // either the scratch buffer or the caller's output (free until the last pass), chosen
-    // backwards from the last pass so that no pass reads and writes the same buffer and
-    // the last pass reads scratch and writes rowind / cscval.
-    const int passes = radix_passes(N);
-    const int *src_k = colind;
-    const int *src_r = rowidx;
-    const unsigned *src_v = perm ? nullptr : reinterpret_cast<const unsigned *>(val);
-    for (int pass = 0; pass < passes; ++pass) {
-        const bool last = pass == passes - 1;
-        const bool to_scratch = ((passes - 1 - pass) & 1) != 0;
-        int *dk = (pass & 1) ? keysB : keysA;
-        int *dr = (last || !to_scratch) ? rowind : rowsT;
-        unsigned *dv = wv ? ((last || !to_scratch) ? final_v : valsT) : nullptr;
-        const int shift = 8 * pass;
-        radix_histogram<<<tiles, kThreads, 0, s>>>(src_k, nnz, shift, tiles, N, hist,
-                                                   ctx->d_status, pass == 0);
-        ctx->launches++;
-        as_status st = exclusive_scan(ctx, hist, hist, hist_n, sums, s);
-        if (st != AS_OK) return st;
-        radix_scatter<<<tiles, kThreads, 0, s>>>(src_k, src_r, src_v, perm && pass == 0, nnz,
-                                                 shift, tiles, hist, dk, dr, dv);
-        ctx->launches++;
-        src_k = dk;
-        src_r = dr;
-        src_v = dv;
-    }
-    colptr_from_keys<<<static_cast<unsigned>(ceil_div(static_cast<long>(nnz) + 1, kThreads)),
-                       kThreads, 0, s>>>(src_k, nnz, N, colptr);
-    ctx->launches++;
+    SortBuffers w;
+    w.keysA = reinterpret_cast<int *>(take(sizeof(int) * static_cast<size_t>(nnz)));
+    w.keysB = reinterpret_cast<int *>(take(sizeof(int) * static_cast<size_t>(nnz)));
+    w.rowsT = reinterpret_cast<int *>(take(sizeof(int) * static_cast<size_t>(nnz)));
+    w.valsT = wv ? reinterpret_cast<unsigned *>(take(sizeof(unsigned) * static_cast<size_t>(nnz))) : nullptr;
+    w.hist = reinterpret_cast<int *>(take(sizeof(int) * static_cast<size_t>(hist_n)));
+    w.sums = reinterpret_cast<int *>(take(sizeof(int) * static_cast<size_t>(ceil_div(hist_n, kScanChunk) + 1)));
+    ctx->launches += sort_by_column(M, N, nnz, rowptr, colind,
+                                    perm ? nullptr : reinterpret_cast<const unsigned *>(val),
+                                    perm != nullptr, colptr, rowind, final_v, w, ctx->d_status, s);
     return check_cuda(cudaGetLastError(), "csr2csc launch");
 }
 
@@ -515,10 +682,12 @@ namespace as {
 namespace {
 
 constexpr size_t align256c(size_t b) { return (b + 255) & ~size_t(255); }
-constexpr long kStaticTiles = (AS_CSR2CSC_STATIC_MAX_NNZ + kTile - 1) / kTile;
+constexpr long kStaticTile = kSortThreads * kSmallItems;
+static_assert(AS_CSR2CSC_STATIC_MAX_NNZ < kLargeNnz, "small tiles only");
+constexpr long kStaticTiles = (AS_CSR2CSC_STATIC_MAX_NNZ + kStaticTile - 1) / kStaticTile;
 constexpr long kStaticHist = kStaticTiles * kBins;
 constexpr size_t kStaticScratchBytes =
-    5 * align256c(sizeof(int) * static_cast<size_t>(AS_CSR2CSC_STATIC_MAX_NNZ)) +
+    4 * align256c(sizeof(int) * static_cast<size_t>(AS_CSR2CSC_STATIC_MAX_NNZ)) +
     align256c(sizeof(int) * static_cast<size_t>(kStaticHist)) +
     align256c(sizeof(int) * static_cast<size_t>((kStaticHist + kScanChunk - 1) / kScanChunk + 1));
 constexpr int kStaticMaxDevices = 64;
@@ -560,49 +729,17 @@ cudaError_t static_slot(int dev, StaticSlot *out) {
 cudaError_t csr2csc_static_run(int M, int N, int nnz, const int *rowptr, const int *colind,
                                const float *val, int *colptr, int *rowind, float *cscval,
                                unsigned char *work, unsigned *status, cudaStream_t s) {
-    const bool wv = val != nullptr;
-    const int tiles = static_cast<int>(ceil_div(nnz, kTile));
-    const long hist_n = static_cast<long>(tiles) * kBins;
     const size_t cap = align256c(sizeof(int) * static_cast<size_t>(AS_CSR2CSC_STATIC_MAX_NNZ));
-    int *rowidx = reinterpret_cast<int *>(work);
-    int *keysA = reinterpret_cast<int *>(work + cap);
-    int *keysB = reinterpret_cast<int *>(work + 2 * cap);
-    int *rowsT = reinterpret_cast<int *>(work + 3 * cap);
-    float *valsT = reinterpret_cast<float *>(work + 4 * cap);
-    int *hist = reinterpret_cast<int *>(work + 5 * cap);
-    int *sums = reinterpret_cast<int *>(work + 5 * cap + align256c(sizeof(int) * kStaticHist));
-
-    const unsigned gw = static_cast<unsigned>(ceil_div(ceil_div(nnz, kExpand), kThreads));
-    expand_rows<<<gw, kThreads, 0, s>>>(M, nnz, rowptr, rowidx, status);
-    const long cb = ceil_div(nnz, kThreads);
-    check_rowptr_ends<<<static_cast<unsigned>(cb < 4096 ? cb : 4096), kThreads, 0, s>>>(
-        M, nnz, rowptr, rowidx, status);
-    const int passes = radix_passes(N);
-    const int *src_k = colind;
-    const int *src_r = rowidx;
-    const unsigned *src_v = reinterpret_cast<const unsigned *>(val);  // value bits, moved as is
-    const long nb = ceil_div(hist_n, kScanChunk);
-    for (int pass = 0; pass < passes; ++pass) {
-        const bool last = pass == passes - 1;
-        const bool to_scratch = ((passes - 1 - pass) & 1) != 0;
-        int *dk = (pass & 1) ? keysB : keysA;
-        int *dr = (last || !to_scratch) ? rowind : rowsT;
-        unsigned *dv = wv ? reinterpret_cast<unsigned *>((last || !to_scratch) ? cscval : valsT)
-                          : nullptr;
-        const int shift = 8 * pass;
-        radix_histogram<<<tiles, kThreads, 0, s>>>(src_k, nnz, shift, tiles, N, hist, status,
-                                                   pass == 0);
-        scan_reduce<<<static_cast<unsigned>(nb), kThreads, 0, s>>>(hist, hist_n, sums);
-        scan_block_sums<<<1, kThreads, 0, s>>>(sums, static_cast<int>(nb));
-        scan_downsweep<<<static_cast<unsigned>(nb), kThreads, 0, s>>>(hist, hist_n, sums, hist);
-        radix_scatter<<<tiles, kThreads, 0, s>>>(src_k, src_r, src_v, false, nnz, shift, tiles,
-                                                 hist, dk, dr, dv);
-        src_k = dk;
-        src_r = dr;
-        src_v = dv;
-    }
-    colptr_from_keys<<<static_cast<unsigned>(ceil_div(static_cast<long>(nnz) + 1, kThreads)),
-                       kThreads, 0, s>>>(src_k, nnz, N, colptr);
+    SortBuffers w;
+    w.keysA = reinterpret_cast<int *>(work);
+    w.keysB = reinterpret_cast<int *>(work + cap);
+    w.rowsT = reinterpret_cast<int *>(work + 2 * cap);
+    w.valsT = reinterpret_cast<unsigned *>(work + 3 * cap);
+    w.hist = reinterpret_cast<int *>(work + 4 * cap);
+    w.sums = reinterpret_cast<int *>(work + 4 * cap + align256c(sizeof(int) * kStaticHist));
+    (void)sort_by_column(M, N, nnz, rowptr, colind, reinterpret_cast<const unsigned *>(val), false,
+                         colptr, rowind, val ? reinterpret_cast<unsigned *>(cscval) : nullptr, w,
+                         status, s);
     return cudaGetLastError();
 }
 
