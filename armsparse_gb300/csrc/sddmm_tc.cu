@@ -311,7 +311,8 @@ sddmm_tc_kernel(const __grid_constant__ CUtensorMap tmXhi, const __grid_constant
 // One CTA per SM walks the tiles (grouped order: 16 row tiles at a time across all column
 // tiles, for L2 reuse of the operand panels) and skips tiles without pattern entries (a
 // pre-pass marks them). Two accumulators in tensor memory (2 x BN columns): the epilogue
-// warps drain tile j from one while the MMA thread accumulates tile j+1 in the other. BK is
+// warps drain tile j from one while the MMA thread accumulates tile j+1 in the other. BN is the
+// tile's width (tile_width picks it). BK is
 // the K width of a pipeline stage: 64 (128-byte swizzle, 2 stages of 96 KB) or 32 (64-byte
 // swizzle, 4 stages of 48 KB).
 template <int BN, int BK>
@@ -324,6 +325,7 @@ struct PSmem {
     static constexpr int kBytes = 1024 + kStages * kStage + kStaging + 512;
     static constexpr int kLayout = BK == 32 ? 4 : 2;  // descriptor swizzle: 64B / 128B
     static constexpr int kSBO = 8 * BK * 2;           // bytes between 8-row core groups
+    static constexpr int kAccCols = BN <= 128 ? 128 : 256;  // tensor memory columns per accumulator
 };
 constexpr int kGroupM = 16;
 
@@ -385,7 +387,7 @@ sddmm_tc_persistent(const __grid_constant__ CUtensorMap tmXhi, const __grid_cons
     if (warp == 1) {
         asm volatile("tcgen05.alloc.cta_group::1.sync.aligned.shared::cta.b32 [%0], %1;" ::"r"(
                          smem_u32(tmem_slot)),
-                     "r"(2 * BN)
+                     "r"(2 * L::kAccCols)
                      : "memory");
         asm volatile("tcgen05.relinquish_alloc_permit.cta_group::1.sync.aligned;" ::: "memory");
     }
@@ -432,7 +434,7 @@ sddmm_tc_persistent(const __grid_constant__ CUtensorMap tmXhi, const __grid_cons
                 const int buf = j & 1, use = j >> 1;
                 if (use > 0 && !mbar_wait(&acce[buf], (use - 1) & 1, abort_flag, status)) break;
                 tc_fence_after();
-                const uint32_t d = tmem + buf * BN;
+                const uint32_t d = tmem + buf * L::kAccCols;
                 for (int kb = 0; kb < nkb; ++kb, ++it) {
                     const int s = it % L::kStages, r = it / L::kStages;
                     if (!mbar_wait(&full[s], r & 1, abort_flag, status)) {
@@ -493,7 +495,7 @@ sddmm_tc_persistent(const __grid_constant__ CUtensorMap tmXhi, const __grid_cons
 #pragma unroll 1
             for (int jj = 0; jj < BN / 32; ++jj) {
                 uint32_t v[32];
-                tmem_ld32(lane_addr + buf * BN + 32 * jj, v);
+                tmem_ld32(lane_addr + buf * L::kAccCols + 32 * jj, v);
                 const int cend = c0 + 32 * (jj + 1);
                 if (e < hi && __ldg(colind + e) < cend) {
 #pragma unroll
@@ -522,7 +524,7 @@ sddmm_tc_persistent(const __grid_constant__ CUtensorMap tmXhi, const __grid_cons
     __syncthreads();
     if (warp == 1) {
         tc_fence_after();
-        asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, %1;" ::"r"(tmem), "r"(2 * BN)
+        asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, %1;" ::"r"(tmem), "r"(2 * L::kAccCols)
                      : "memory");
     }
 }
@@ -538,7 +540,7 @@ sddmm_tc_persistent(const __grid_constant__ CUtensorMap tmXhi, const __grid_cons
 constexpr int kMarkSharedTiles = 16384;  // tiles per band held in shared memory
 
 template <bool SHARED>
-__global__ void __launch_bounds__(256)
+__device__ __forceinline__ void
 check_and_mark(int M, int N, int nnz, const int *__restrict__ rowptr,
                const int *__restrict__ colind, int BN, int tiles_n, unsigned char *__restrict__ occ,
                unsigned *status) {
@@ -590,15 +592,16 @@ check_and_mark(int M, int N, int nnz, const int *__restrict__ rowptr,
 
 // X's rows then Y's rows -> bf16 hi/lo planes: hi = bf16(x), lo = bf16(x - hi), columns
 // [K, Kp) zero. A block takes (row, 4096-column segment) items; each thread issues its four
-// 16-byte loads before converting, so a block keeps 16 KB of loads in flight.
-__global__ void __launch_bounds__(256)
-split_xy(long M, long N, int K, int Kp, const float *__restrict__ X, long ldx, bool vx,
+// 16-byte loads before converting, so a block keeps 16 KB of loads in flight. Block `block` of
+// `blocks`.
+__device__ __forceinline__ void
+split_rows(long block, long blocks, long M, long N, int K, int Kp, const float *__restrict__ X, long ldx, bool vx,
          const float *__restrict__ Y, long ldy, bool vy, uint16_t *__restrict__ xhi,
          uint16_t *__restrict__ xlo, uint16_t *__restrict__ yhi, uint16_t *__restrict__ ylo) {
     constexpr int kSeg = 4096;
     const long segs = (Kp + kSeg - 1) / kSeg;
     const long items = (M + N) * segs;
-    for (long item = blockIdx.x; item < items; item += gridDim.x) {
+    for (long item = block; item < items; item += blocks) {
         const long row = item / segs;
         const int base = static_cast<int>(item - row * segs) * kSeg;
         const bool isx = row < M;
@@ -636,8 +639,38 @@ split_xy(long M, long N, int K, int Kp, const float *__restrict__ X, long ldx, b
     }
 }
 
-// hi = bf16(x), lo = bf16(x - hi); columns [K, Kp) are zero. Blocks stride over rows,
-// threads over groups of four columns.
+struct SplitArgs {
+    long M, N;
+    int K, Kp;
+    const float *X;
+    long ldx;
+    bool vx;
+    const float *Y;
+    long ldy;
+    bool vy;
+    uint16_t *xhi, *xlo, *yhi, *ylo;
+};
+__device__ __forceinline__ void split_rows(long block, long blocks, const SplitArgs &a) {
+    split_rows(block, blocks, a.M, a.N, a.K, a.Kp, a.X, a.ldx, a.vx, a.Y, a.ldy, a.vy, a.xhi, a.xlo,
+               a.yhi, a.ylo);
+}
+__global__ void __launch_bounds__(256) split_xy(SplitArgs a) {
+    split_rows(blockIdx.x, gridDim.x, a);
+}
+
+// The pattern check and tile marks (blocks below mark_blocks) and the split in one launch: neither
+// needs the other, and the marks' latency hides under the split's stream (4096 x 4096, density
+// 0.1: 10.8 + 47.5 us as two launches, 52.4 as one).
+template <bool SHARED>
+__global__ void __launch_bounds__(256)
+mark_and_split(unsigned mark_blocks, int M, int N, int nnz, const int *__restrict__ rowptr,
+               const int *__restrict__ colind, int BN, int tiles_n, unsigned char *__restrict__ occ,
+               unsigned *status, SplitArgs a) {
+    if (blockIdx.x < mark_blocks)  // the same for the whole block
+        check_and_mark<SHARED>(M, N, nnz, rowptr, colind, BN, tiles_n, occ, status);
+    else
+        split_rows(blockIdx.x - mark_blocks, gridDim.x - mark_blocks, a);
+}
 
 // Columns must ascend within rows for the tile walk; flag rows that break it (one warp per
 // row, coalesced).
@@ -746,6 +779,25 @@ as_status launch_persistent(as_ctx *ctx, int M, int N, int Kp, int nnz, const in
 
 int sddmm_tc_variant_count() { return 3; }
 
+// Width of the persistent kernel's tiles: the one that takes the least time when its 128 x BN
+// tiles run in whole waves over the SMs, a tile's time being its MMAs (BN) and the part of it
+// that does not shrink with it (32 columns' worth). 4096 x 4096 on 152 SMs: 256-wide tiles leave
+// 56 of 512 to a fourth wave, 608 of 224 columns make four full
+// ones: 240 against 276 us (K = 4096).
+static int tile_width(int M, int N, int sms) {
+    int best = 256;
+    long best_cost = 0;
+    for (int w = 256; w >= 128; w -= 32) {
+        const long tiles = ceil_div(M, kBM) * ceil_div(N, w);
+        const long cost = ceil_div(tiles, sms) * (w + 32);
+        if (best_cost == 0 || cost < best_cost) {
+            best = w;
+            best_cost = cost;
+        }
+    }
+    return best;
+}
+
 // variant: 1 = one tile per CTA (K block 64), 2 = persistent, K block 64, 3 = persistent,
 // K block 32 (deeper pipeline); 0 = library choice.
 as_status sddmm_bf16x3_launch(as_ctx *ctx, int M, int N, int K, int nnz, const int *rowptr,
@@ -753,7 +805,7 @@ as_status sddmm_bf16x3_launch(as_ctx *ctx, int M, int N, int K, int nnz, const i
                               const float *Y, long ldy, float *out, int variant, cudaStream_t s) {
     if (variant == 0) variant = 3;  // persistent, 4-stage pipeline: fastest on GB300
     if (M == 0) return fail(AS_ERR_INVALID_CSR, "sddmm: nnz > 0 with zero rows");
-    const int BN = 256;
+    const int BN = variant == 3 ? tile_width(M, N, ctx->sms) : 256;
     const int Kp = static_cast<int>(ceil_div(K, kBK) * kBK);
     const size_t xs = static_cast<size_t>(M) * Kp * 2, ys = static_cast<size_t>(N) * Kp * 2;
     auto al = [](size_t b) { return (b + 1023) & ~size_t(1023); };
@@ -765,19 +817,11 @@ as_status sddmm_bf16x3_launch(as_ctx *ctx, int M, int N, int K, int nnz, const i
     uint8_t *p = static_cast<uint8_t *>(w);
     unsigned char *occ = p + 2 * al(xs) + 2 * al(ys);
     const unsigned rows_grid = static_cast<unsigned>(ceil_div(static_cast<long>(M) * 32, 256));
-    if (variant == 1 || K == 0) {
+    const bool marks = variant != 1 && K > 0;
+    if (!marks) {
         check_sorted_rows<<<rows_grid, 256, 0, s>>>(M, N, nnz, rowptr, colind, ctx->d_status);
-    } else {
-        cudaError_t e = cudaMemsetAsync(occ, 0, occ_bytes, s);
-        if (e != cudaSuccess) return check_cuda(e, "sddmm_bf16x3: occupancy clear");
-        if (tiles_n <= kMarkSharedTiles)
-            check_and_mark<true><<<rows_grid, 256, static_cast<size_t>(tiles_n), s>>>(
-                M, N, nnz, rowptr, colind, BN, tiles_n, occ, ctx->d_status);
-        else
-            check_and_mark<false><<<rows_grid, 256, 0, s>>>(M, N, nnz, rowptr, colind, BN,
-                                                            tiles_n, occ, ctx->d_status);
+        ctx->launches++;
     }
-    ctx->launches++;
     if (K == 0) {
         fill_zero<<<static_cast<unsigned>(ceil_div(nnz, 256) < 4096 ? ceil_div(nnz, 256) : 4096), 256, 0, s>>>(out, nnz);
         ctx->launches++;
@@ -791,16 +835,34 @@ as_status sddmm_bf16x3_launch(as_ctx *ctx, int M, int N, int K, int nnz, const i
     const bool vy = ldy % 4 == 0 && reinterpret_cast<uintptr_t>(Y) % 16 == 0;
     const long items = (static_cast<long>(M) + N) * ceil_div(Kp, 4096);
     const unsigned sg = static_cast<unsigned>(items < 152L * 8 ? items : 152L * 8);
-    split_xy<<<sg, 256, 0, s>>>(M, N, K, Kp, X, ldx, vx, Y, ldy, vy, xhi, xlo, yhi, ylo);
+    const SplitArgs sp{M, N, K, Kp, X, ldx, vx, Y, ldy, vy, xhi, xlo, yhi, ylo};
+    if (marks) {
+        cudaError_t e = cudaMemsetAsync(occ, 0, occ_bytes, s);
+        if (e != cudaSuccess) return check_cuda(e, "sddmm_bf16x3: occupancy clear");
+        if (tiles_n <= kMarkSharedTiles)
+            mark_and_split<true><<<rows_grid + sg, 256, static_cast<size_t>(tiles_n), s>>>(
+                rows_grid, M, N, nnz, rowptr, colind, BN, tiles_n, occ, ctx->d_status, sp);
+        else
+            mark_and_split<false><<<rows_grid + sg, 256, 0, s>>>(
+                rows_grid, M, N, nnz, rowptr, colind, BN, tiles_n, occ, ctx->d_status, sp);
+    } else {
+        split_xy<<<sg, 256, 0, s>>>(sp);
+    }
     ctx->launches++;
     st = check_cuda(cudaGetLastError(), "sddmm_bf16x3 split");
     if (st != AS_OK) return st;
     if (variant == 2)
         return launch_persistent<256, 64>(ctx, M, N, Kp, nnz, rowptr, colind, aval, out, xhi, xlo,
                                           yhi, ylo, occ, s);
-    if (variant == 3)
-        return launch_persistent<256, 32>(ctx, M, N, Kp, nnz, rowptr, colind, aval, out, xhi, xlo,
-                                          yhi, ylo, occ, s);
+    if (variant == 3) {
+#define AS_TC_WIDTH(W)                                                                            \
+    case W:                                                                                       \
+        return launch_persistent<W, 32>(ctx, M, N, Kp, nnz, rowptr, colind, aval, out, xhi, xlo,  \
+                                        yhi, ylo, occ, s);
+        switch (BN) { AS_TC_WIDTH(128) AS_TC_WIDTH(160) AS_TC_WIDTH(192) AS_TC_WIDTH(224) AS_TC_WIDTH(256) }
+#undef AS_TC_WIDTH
+        return fail(AS_ERR_UNSUPPORTED, "sddmm_bf16x3: tile width");
+    }
     return launch_tiles<256>(ctx, M, N, Kp, nnz, rowptr, colind, aval, out, xhi, xlo, yhi, ylo, s);
 }
 
