@@ -83,6 +83,25 @@ __device__ __forceinline__ void row_range(const int *rowptr, int r, int nnz, uns
     }
 }
 
+// The row that holds entry e (largest r with rowptr[r] <= e), searched by a group of GROUP lanes:
+// each step probes GROUP points at once, so 2^21 rows take five dependent loads with 32 lanes,
+// not 21. Always in [0, M), whatever rowptr holds.
+template <int GROUP>
+__device__ __forceinline__ int find_row(const int *__restrict__ rowptr, int M, long e, int g,
+                                        unsigned gmask) {
+    long lo = 0, hi = M;
+    while (hi - lo > 1) {
+        const long width = hi - lo;
+        const long probe = lo + width * (g + 1) / (GROUP + 1);
+        const int c = __popc(__ballot_sync(gmask, __ldg(rowptr + probe) <= e) & gmask);
+        const long nlo = c > 0 ? lo + width * c / (GROUP + 1) : lo;
+        const long nhi = c < GROUP ? lo + width * (c + 1) / (GROUP + 1) : hi;
+        lo = nlo;
+        hi = nhi;
+    }
+    return static_cast<int>(lo);
+}
+
 __host__ __device__ __forceinline__ long long ceil_div(long long a, long long b) {
     return (a + b - 1) / b;
 }

@@ -22,19 +22,6 @@ namespace {
 
 constexpr int kThreads = 256;
 
-__device__ __forceinline__ int find_row(const int *__restrict__ rowptr, int M, long e) {
-    // largest r in [0, M) with rowptr[r] <= e
-    int lo = 0, hi = M;  // invariant: rowptr[lo] <= e < rowptr[hi] for valid CSR
-    while (hi - lo > 1) {
-        const int mid = (lo + hi) >> 1;
-        if (__ldg(rowptr + mid) <= e)
-            lo = mid;
-        else
-            hi = mid;
-    }
-    return lo;
-}
-
 // acc = fma(x0, y0, acc); acc = fma(x1, y1, acc) for the bf16 halves of x and y, in order.
 __device__ __forceinline__ void fma_bf16_seq2(unsigned x, unsigned y, float &acc) {
     asm("{\n .reg .b16 xl, xh, yl, yh;\n mov.b32 {xl, xh}, %1;\n mov.b32 {yl, yh}, %2;\n"
@@ -52,6 +39,13 @@ template <>
 struct Block<float> {
     using Raw = float4;
     __device__ static Raw load(const float *p) { return __ldg(reinterpret_cast<const float4 *>(p)); }
+    __device__ static Raw load_here(const float *p) {
+        Raw v;
+        asm volatile("ld.global.nc.v4.f32 {%0, %1, %2, %3}, [%4];"
+                     : "=f"(v.x), "=f"(v.y), "=f"(v.z), "=f"(v.w)
+                     : "l"(p));
+        return v;
+    }
     __device__ static void chain(const Raw &x, const Raw &y, float &acc) {
         acc = fmaf(x.x, y.x, acc);
         acc = fmaf(x.y, y.y, acc);
@@ -63,6 +57,11 @@ template <>
 struct Block<uint16_t> {
     using Raw = uint2;
     __device__ static Raw load(const uint16_t *p) { return __ldg(reinterpret_cast<const uint2 *>(p)); }
+    __device__ static Raw load_here(const uint16_t *p) {
+        Raw v;
+        asm volatile("ld.global.nc.v2.u32 {%0, %1}, [%2];" : "=r"(v.x), "=r"(v.y) : "l"(p));
+        return v;
+    }
     __device__ static void chain(const Raw &x, const Raw &y, float &acc) {
         fma_bf16_seq2(x.x, y.x, acc);
         fma_bf16_seq2(x.y, y.y, acc);
@@ -127,7 +126,7 @@ sddmm_group(int M, int N, int K, int nnz, int CH, const int *__restrict__ rows,
     const long e1 = e0 + CH < nnz ? e0 + CH : nnz;
     int r = 0, rs = 0, re = 0;
     if (!COO) {
-        r = find_row(rows, M, e0);
+        r = find_row<G>(rows, M, e0, g, gmask);
         rs = __ldg(rows + r);
         re = __ldg(rows + r + 1);
     }
@@ -173,6 +172,74 @@ sddmm_group(int M, int N, int K, int nnz, int CH, const int *__restrict__ rows,
     }
 }
 
+// The CSR form where a lane's part of a row is at most four blocks (K <= 16 G) and rows are
+// aligned: X's row stays in registers while the row lasts, the next edge's Y row is loaded (and
+// the column of the one after it read) while the present edge is summed. The sums are
+// sddmm_group's, in the same order. What bounds it is Y's gathers, so warps in flight count: on a
+// graph of 6M entries with K = 128 it takes 354 us with four CTAs per SM (64 registers), 425 with
+// three, 655 with five (spills); two edges per turn, 488; sddmm_group 461. (K = 512: 1.24 and 2.23
+// ms; K = 16: 0.21 and 0.31.) The loads are volatile because left to the compiler they move down
+// to their uses.
+template <typename T, int G>
+__global__ void __launch_bounds__(kThreads, 4)
+sddmm_rows(int M, int N, int K, int nnz, int CH, const int *__restrict__ rowptr,
+           const int *__restrict__ colind, const float *__restrict__ aval,
+           const T *__restrict__ X, long ldx, const T *__restrict__ Y, long ldy,
+           float *__restrict__ out, unsigned *status) {
+    using B = Block<T>;
+    const long grp = (static_cast<long>(blockIdx.x) * kThreads + threadIdx.x) / G;
+    const int g = threadIdx.x % G;
+    const unsigned gmask =
+        G == 32 ? 0xffffffffu : (((1u << G) - 1u) << ((threadIdx.x & 31) & ~(G - 1)));
+    if (grp * CH >= nnz) return;  // the whole group leaves together
+    const int e0 = static_cast<int>(grp * CH);
+    const int e1 = CH < nnz - e0 ? e0 + CH : nnz;
+    const int nq = K >> 2;
+    int r = find_row<G>(rowptr, M, e0, g, gmask);
+    int rs = __ldg(rowptr + r), re = __ldg(rowptr + r + 1);
+    auto load = [&](const T *row, typename B::Raw (&v)[4]) {
+#pragma unroll
+        for (int u = 0; u < 4; ++u)
+            if (g + u * G < nq) v[u] = B::load_here(row + 4 * (g + u * G));
+    };
+    auto column = [&](int e) { return e < e1 ? ld_stream(colind + e) : -1; };
+    auto in_range = [&](int c) { return static_cast<unsigned>(c) < static_cast<unsigned>(N); };
+    typename B::Raw x[4], y[4], yn[4];
+    int held = -1;  // the row that x holds
+    int c = column(e0), cn = column(e0 + 1);
+    if (in_range(c)) load(Y + c * ldy, y);
+    for (int e = e0; e < e1; ++e) {  // every branch below is the same for the whole group
+        while (e >= re && r + 1 < M) {
+            ++r;
+            rs = re;
+            re = __ldg(rowptr + r + 1);
+        }
+        if (in_range(cn)) load(Y + cn * ldy, yn);
+        const int cnn = column(e + 2);
+        const bool row_ok = rs <= e && re > e;
+        if (row_ok && in_range(c)) {
+            if (held != r) {
+                load(X + r * ldx, x);
+                held = r;
+            }
+            float acc = 0.0f;
+#pragma unroll
+            for (int u = 0; u < 4; ++u)
+                if (g + u * G < nq) B::chain(x[u], y[u], acc);
+#pragma unroll
+            for (int off = G / 2; off > 0; off >>= 1) acc += __shfl_xor_sync(gmask, acc, off, G);
+            if (g == 0) out[e] = aval ? __ldg(aval + e) * acc : acc;
+        } else if (g == 0) {
+            flag(status, row_ok ? kFlagBadColind : kFlagBadRowptr);
+            out[e] = 0.0f;
+        }
+        c = cn;
+        cn = cnn;
+#pragma unroll
+        for (int u = 0; u < 4; ++u) y[u] = yn[u];
+    }
+}
+
 int group_size(int K) {  // the oracle's or_sddmm_group_size: about four blocks per lane
     const int q = (K + 15) / 16;
     int g = 1;
@@ -190,12 +257,23 @@ as_status launch_group(as_ctx *ctx, int M, int N, int K, int nnz, const int *row
                      reinterpret_cast<uintptr_t>(X) % (4 * esz) == 0 &&
                      reinterpret_cast<uintptr_t>(Y) % (4 * esz) == 0;
     const int G = group_size(K);
-    const int CH = G >= 32 ? 4 : 128 / G;  // edges per group: more for short dot products
+    // K in (0, 16 G]: every lane's blocks fit its registers
+    const bool resident = !COO && vec && K > 0 && K <= 16 * G && N > 0;
+    int CH = G >= 32 ? 4 : 128 / G;  // edges per group: more for short dot products
+    if (resident) {  // as many as leave two waves of full SMs, 4 to 64
+        const long all = static_cast<long>(nnz) * G / (2L * 2048 * ctx->sms);
+        CH = static_cast<int>(all < 4 ? 4 : all > 64 ? 64 : all);
+    }
     const long groups = ceil_div(nnz, CH);
     const unsigned grid = static_cast<unsigned>(ceil_div(groups * G, kThreads));
 #define AS_SDDMM_G(GV)                                                                      \
     case GV:                                                                                \
-        if (vec)                                                                            \
+        if (resident) {                                                                     \
+            if constexpr (!COO)                                                             \
+                sddmm_rows<T, GV><<<grid, kThreads, 0, s>>>(M, N, K, nnz, CH, rows, colind, \
+                                                            aval, X, ldx, Y, ldy, out,      \
+                                                            ctx->d_status);                 \
+        } else if (vec)                                                                            \
             sddmm_group<T, true, GV, COO><<<grid, kThreads, 0, s>>>(                        \
                 M, N, K, nnz, CH, rows, colind, aval, X, ldx, Y, ldy, out, ctx->d_status);  \
         else                                                                                \

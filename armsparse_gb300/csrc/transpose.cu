@@ -174,22 +174,6 @@ __device__ __forceinline__ int block_max_scan(int v, int *smem_warp) {
     return v;
 }
 
-// Largest r in [0, M) with rowptr[r] <= e, by a whole warp (32 probes per step).
-__device__ __forceinline__ int warp_find_row(int M, const int *__restrict__ rowptr, long e) {
-    const int lane = threadIdx.x & 31;
-    long lo = 0, hi = M;
-    while (hi - lo > 1) {
-        const long width = hi - lo;
-        const long probe = lo + width * (lane + 1) / 33;
-        const int c = __popc(__ballot_sync(0xffffffffu, __ldg(rowptr + probe) <= e));
-        const long nlo = c > 0 ? lo + width * c / 33 : lo;
-        const long nhi = c < 32 ? lo + width * (c + 1) / 33 : hi;
-        lo = nlo;
-        hi = nhi;
-    }
-    return static_cast<int>(lo);
-}
-
 template <int ITEMS>
 __global__ void __launch_bounds__(kSortThreads)
 radix_histogram(const int *__restrict__ keys, int nnz, int shift, int bins, int tiles, int N,
@@ -274,7 +258,7 @@ radix_scatter(const int *__restrict__ keys, const int *__restrict__ rows,
         const bool ends = __ldg(rowptr) == 0 && __ldg(rowptr + M) == nnz;
         if (!ends && tid == 0 && blockIdx.x == 0) flag(status, kFlagBadRowptr);
         if (warp < 2) {
-            const int r = warp_find_row(M, rowptr, warp == 0 ? base : base + n_tile - 1);
+            const int r = find_row<32>(rowptr, M, warp == 0 ? base : base + n_tile - 1, lane, 0xffffffffu);
             if (lane == 0) row_span[warp] = r;
         }
         for (int i = tid; i < kTile; i += kSortThreads) sr[i] = 0;
