@@ -91,6 +91,8 @@ class NativeError(RuntimeError):
 def load(path: str | None = None) -> ctypes.CDLL:
     """Load the C-ABI library (raises if it is absent: there is no CPU fallback)."""
     global _lib
+    if _lib is not None:  # the lock is for the first call only
+        return _lib
     with _lock:
         if _lib is None:
             p = path or LIB_PATH

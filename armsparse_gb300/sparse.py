@@ -14,26 +14,31 @@ def _ptr(t: torch.Tensor | None):
 
 
 def _stream(device: torch.device) -> int:
-    return torch.cuda.current_stream(device).cuda_stream
+    # the raw handle of torch's current stream, without building a Stream object for it
+    index = device.index
+    return torch._C._cuda_getCurrentRawStream(torch.cuda.current_device() if index is None else index)
 
 
 def _dev(*ts) -> torch.device:
-    dev = None
+    first, index = None, -1
     for t in ts:
         if t is None:
             continue
-        if not t.is_cuda:
+        i = t.get_device() if t.is_cuda else -1
+        if i < 0:
             raise ValueError("armsparse_gb300 works on CUDA tensors only (no CPU path)")
-        if dev is None:
-            dev = t.device
-        elif t.device != dev:
+        if first is None:
+            first, index = t, i
+        elif i != index:
             raise ValueError("all tensors must be on the same device")
-    if dev is None:
+    if first is None:
         raise ValueError("no tensor given")
-    return dev
+    return first.device
 
 
 def _need(t: torch.Tensor, dtype, name: str, ndim: int | None = None):
+    if t.dtype is dtype and t.is_contiguous() and (ndim is None or t.dim() == ndim):
+        return
     if t.dtype != dtype:
         raise TypeError(f"{name} must be {dtype}, got {t.dtype}")
     if not t.is_contiguous():
