@@ -30,9 +30,10 @@
 //    segments (all kBlk in flight; the indices were loaded one turn earlier), 16 bytes per lane
 //    and four entries per load where the layout allows, waits until the slot's last block has
 //    been consumed, and stores segments and values (word c of a segment belongs to consumer
-//    lane c % 4 * 8 + c / 4, which makes these stores free of bank conflicts). Positions that add nothing (past a row's end, or entries a row-pair unit leaves
-//    out) get the word -0.0 and the value 1, which keep every accumulator as it is, so the
-//    consumer runs one form of the step.
+//    lane c % 4 * 8 + c / 4, which makes these stores free of bank conflicts). Positions that
+//    add nothing (past a row's end, or entries a row-pair unit leaves out) get the word -0.0 and
+//    the value 1, which keep every accumulator as it is, so the consumer runs one form of the
+//    step.
 // The consumer shares its SM sub-partition with an idle warp only (warp 4): the chain issues
 // one step every four cycles and loses a share of that rate to every busy neighbour.
 //

@@ -14,10 +14,11 @@
 //                          first output slot;
 //   3. stable scatter   -- each warp of a CTA ranks the entries of its own consecutive part of
 //                          the tile among equal digits before them (a ballot per bit finds
-//                          the lanes of a digit, a warp-private count those before them), one scan over warps and digits turns
-//                          ranks into slots of the tile, the tile is parked in shared memory
-//                          sorted by digit, then key, row and value are written out in that
-//                          order, so each digit's entries leave as one coalesced run.
+//                          the lanes of a digit, a warp-private count those before them),
+//                          one scan over warps and digits turns ranks into slots of the tile,
+//                          the tile is parked in shared memory sorted by digit, then key, row
+//                          and value are written out in that order, so each digit's entries
+//                          leave as one coalesced run.
 // The first pass works out each entry's row from the row pointer as it goes (each row marks its
 // first entry in the tile, a running maximum gives the rest), so row ids are never written and
 // read just to be sorted.
