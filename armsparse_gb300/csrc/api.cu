@@ -46,15 +46,20 @@ as_status scratch(as_ctx *ctx, size_t bytes, void **out) {
 as_status scratch_list(as_ctx *ctx, long n, cudaStream_t s, int **out) {
     const size_t bytes = static_cast<size_t>(n) * sizeof(int);
     *out = nullptr;
-    if (bytes > ctx->scratch_bytes) {
-        cudaStreamCaptureStatus cap = cudaStreamCaptureStatusNone;
-        if (cudaStreamIsCapturing(s, &cap) != cudaSuccess || cap != cudaStreamCaptureStatusNone)
-            return AS_OK;
-    }
+    if (!scratch_fits(ctx, bytes, s)) return AS_OK;
     void *p = nullptr;
     const as_status st = scratch(ctx, bytes, &p);
     if (st == AS_OK) *out = static_cast<int *>(p);
     return st;
+}
+
+bool scratch_fits(as_ctx *ctx, size_t bytes, cudaStream_t s) {
+    if (bytes <= ctx->scratch_bytes) return true;
+    cudaStreamCaptureStatus cap = cudaStreamCaptureStatusNone;
+    if (cudaStreamIsCapturing(s, &cap) != cudaSuccess || cap != cudaStreamCaptureStatusNone)
+        return false;
+    void *p = nullptr;
+    return scratch(ctx, bytes, &p) == AS_OK;
 }
 
 struct DeviceGuard {

@@ -37,9 +37,14 @@ as_status check_cuda(cudaError_t e, const char *what);
 // pointer that earlier work still holds.
 as_status scratch(as_ctx *ctx, size_t bytes, void **out);
 
-// A scratch list of n ints, or nullptr (and AS_OK) when the arena would have to grow while the
-// stream is being captured: the caller then runs without a list.
+// A scratch list of n ints, or nullptr (and AS_OK) when the arena cannot hold it (see
+// scratch_fits): the caller then runs without a list.
 as_status scratch_list(as_ctx *ctx, long n, cudaStream_t s, int **out);
+// Whether the arena holds `bytes`, grown for it where that can be done (a call that is being
+// captured cannot grow it).
+bool scratch_fits(as_ctx *ctx, size_t bytes, cudaStream_t s);
+// The scratch of an entry-balanced SpMM: carry slots and row marks of its chunks.
+size_t spmm_nnz_scratch(int nnz, int N, int chunk);
 
 // ---- launchers (return AS_OK or an error; count launches in ctx) ----
 struct SpmmArgs {

@@ -517,11 +517,13 @@ as_status spmm_launch(as_ctx *ctx, int dtype, int variant, const SpmmArgs &a, cu
 // that bring several entries per load (35.8M entries, width 48, bf16: 2.55 ms with one entry per
 // warp step, 1.66 with two). Each class lists the narrowest tile first; a layout that none of a class
 // serves takes the 1024-entry kernels with 4- and 16-byte vectors, and one that those do not serve
-// is refused.
+// is refused. Shorter chunks leave more carry slots: where the arena cannot hold them (the call is
+// being captured, or memory is short), the 1024-entry kernel runs.
 struct FusedPick {
     int kind, vb, group, cpl, chunk, steps;
 };
-static int fused_default(int dtype, const SpmmArgs &a, const SddmmFuse &f) {
+static int fused_default(as_ctx *ctx, int dtype, const SpmmArgs &a, const SddmmFuse &f,
+                         cudaStream_t s) {
     const int esz = dtype == 0 ? 4 : 2;
     const Variant *t = dtype == 0 ? kF32 : kBF16;
     const int n = spmm_variant_count(dtype);
@@ -556,7 +558,7 @@ static int fused_default(int dtype, const SpmmArgs &a, const SddmmFuse &f) {
     if (fallback == 0) return 0;  // layouts that the fused pass does not serve
     const int v = a.nnz >= 5000000 ? first(large, 5)
                   : a.nnz >= 300000 ? first(medium, 4) : first(small, 5);
-    return v ? v : fallback;
+    return v && scratch_fits(ctx, spmm_nnz_scratch(a.nnz, a.N, t[v - 1].unroll), s) ? v : fallback;
 }
 
 // The SpMM with the SDDMM fused in (spmm_nnz.cu): nnz-split and multi-entry variants, one column
@@ -567,7 +569,7 @@ as_status spmm_sddmm_launch(as_ctx *ctx, int dtype, int variant, const SpmmArgs 
     const Variant *t = dtype == 0 ? kF32 : kBF16;
     auto tile = [&](const Variant &v) { return (v.vb / esz) * v.group * v.cpl; };
     if (variant == 0) {
-        variant = fused_default(dtype, a, f);
+        variant = fused_default(ctx, dtype, a, f, s);
         if (variant == 0)
             return fail(AS_ERR_UNSUPPORTED, "spmm+sddmm: no variant covers this N and layout");
     }

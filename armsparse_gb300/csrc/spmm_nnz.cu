@@ -690,6 +690,10 @@ spmm_empty_rows(int M, int N, const int *__restrict__ rowptr, float *__restrict_
     }
 }
 
+size_t carry_size(long nchunks, int N) {
+    return (sizeof(float) * static_cast<size_t>(2 * nchunks) * N + 255) & ~size_t(255);
+}
+
 // ME: the multi-entry kernel (spmm_nnzme, CPL 1); else spmm_nnzsplit.
 template <typename T, int VB, int G, int CPL, int U, bool FUSE, bool ME = false>
 as_status launch(as_ctx *ctx, const SpmmArgs &a, int CH, const SddmmFuse *fu, cudaStream_t s) {
@@ -710,8 +714,8 @@ as_status launch(as_ctx *ctx, const SpmmArgs &a, int CH, const SddmmFuse *fu, cu
                     "spmm+sddmm: the variant's column tile must cover N, F aligned to its vectors");
     const long nchunks = ceil_div(a.nnz, CH);
     void *w = nullptr;
-    const size_t carry_bytes = (sizeof(float) * static_cast<size_t>(2 * nchunks) * a.N + 255) & ~size_t(255);
-    as_status st = scratch(ctx, carry_bytes + sizeof(int) * static_cast<size_t>(nchunks), &w);
+    const size_t carry_bytes = carry_size(nchunks, a.N);
+    as_status st = scratch(ctx, spmm_nnz_scratch(a.nnz, a.N, CH), &w);
     if (st != AS_OK) return st;
     float *carry = static_cast<float *>(w);
     int *fix = reinterpret_cast<int *>(static_cast<char *>(w) + carry_bytes);
@@ -766,6 +770,11 @@ as_status launch_me(as_ctx *ctx, const SpmmArgs &a, int CH, const SddmmFuse *fu,
 }
 
 }  // namespace
+
+size_t spmm_nnz_scratch(int nnz, int N, int chunk) {
+    const long nchunks = ceil_div(nnz, chunk);
+    return carry_size(nchunks, N) + sizeof(int) * static_cast<size_t>(nchunks);
+}
 
 as_status spmm_nnzme_launch(as_ctx *ctx, int dtype, int vb, int group, int chunk,
                             const SpmmArgs &a, cudaStream_t s, const SddmmFuse *fuse) {

@@ -90,3 +90,26 @@ def test_fused_choice_serves_every_layout(oracle, dtype, N_):
         err = np.abs(dA.cpu().numpy() - (x * y).sum(1))
         assert (err <= 2.0 ** -23 * (N_ + 6) * np.abs(x * y).sum(1)).all()
     A.sync_status()
+
+
+def test_fused_choice_captured_without_room(monkeypatch):
+    """A captured call whose arena holds the 1024-entry kernel's carry slots only runs that kernel."""
+    from armsparse_gb300 import _native
+    ctx = _native.Context(0)
+    monkeypatch.setattr(_native, "context", lambda device=0: ctx)
+    a = S.powerlaw_csr(3000, 2.1, 20.0, 3)
+    B, F = (to_dev(S.dense_uniform((n, 48), s)) for n, s in ((a.n_cols, 1), (a.n_rows, 2)))
+    args = (*csr_dev(a), B, F)
+    long_chunks = A.spmm_variants(torch.float32).index("nnzsplit_v16_g32_c1_ch1024") + 1
+    want, dwant = A.spmm_sddmm(*args, variant=long_chunks)
+    C, dA = torch.empty_like(want), torch.empty_like(dwant)
+    torch.cuda.synchronize()
+    g = torch.cuda.CUDAGraph()
+    with torch.cuda.graph(g):
+        A.spmm_sddmm(*args, C=C, dA=dA)
+    g.replay()
+    torch.cuda.synchronize()
+    assert np.array_equal(bits(C), bits(want)) and np.array_equal(bits(dA), bits(dwant))
+    ctx.sync_status()
+    g.reset()
+    ctx.close()
