@@ -265,7 +265,11 @@ radix_scatter(const int *__restrict__ keys, const int *__restrict__ rows,
         for (int i = tid; i < kTile; i += kSortThreads) sr[i] = 0;
         __syncthreads();
         const int ra = row_span[0], rb = row_span[1];
-        for (long r = static_cast<long>(ra) + tid; r <= rb; r += kSortThreads) {
+        // A tile across a long run of empty rows: each entry looks its row up instead of the CTA
+        // marking them all (10M rows, 1M entries of which the last follows 9M empty rows: 5.0
+        // and 0.12 ms for the call).
+        const bool search = rb - ra > 16 * kTile;
+        for (long r = static_cast<long>(ra) + tid; r <= rb && !search; r += kSortThreads) {
             const long at = static_cast<long>(__ldg(rowptr + r)) - base;
             if (r == ra || (at > 0 && at < n_tile))
                 atomicMax(sr + (r == ra ? 0 : at), static_cast<int>(r));
@@ -291,8 +295,18 @@ radix_scatter(const int *__restrict__ keys, const int *__restrict__ rows,
         for (int i = 0; i < ITEMS; ++i) {
             const int li = w0 + 32 * i;
             if (!ends || li >= n_tile) continue;
-            const int r = sr[li];
             const long e = base + li;
+            int r = sr[li];
+            if (search) {  // the last row of the span that starts at or before the entry
+                r = ra;
+                for (int hi = rb; r < hi;) {
+                    const int mid = r + (hi - r + 1) / 2;
+                    if (__ldg(rowptr + mid) <= e)
+                        r = mid;
+                    else
+                        hi = mid - 1;
+                }
+            }
             const int rs = __ldg(rowptr + r), re = __ldg(rowptr + r + 1);
             if (rs < 0 || re > nnz || e < rs || e >= re)
                 flag(status, kFlagBadRowptr);  // malformed pointers: row 0

@@ -53,3 +53,21 @@ def test_transpose_edges(nnz, cols, kind):
     wide[1:] = cid
     assert np.array_equal(A.csr2csc(rpd, wide[1:], vd, cols)[1].cpu().numpy(), rows)
     A.sync_status()
+
+
+@pytest.mark.parametrize("nnz,gap", [(3000, 16_384), (3000, 16_390), (301_000, 65_536), (301_000, 70_000)])
+def test_transpose_long_runs_of_empty_rows(nnz, gap):
+    """Runs of empty rows inside a tile about as long as where its entries look their rows up."""
+    rng = np.random.default_rng(gap)
+    part = rng.integers(1, 4, 40)
+    lens = np.concatenate([[0] * gap, part, [0] * gap, [1], [0] * (gap - 1), part, [nnz - 2 * part.sum() - 2],
+                           [0] * gap, [1], [0] * gap])
+    rp = np.zeros(lens.size + 1, np.int32)
+    np.cumsum(lens, out=rp[1:])
+    assert rp[-1] == nnz
+    ci = rng.integers(0, 900, nnz).astype(np.int32)
+    order = np.argsort(ci, kind="stable")
+    cp, ri, perm = A.csr2csc_perm(to_dev(rp), to_dev(ci), 900)
+    assert np.array_equal(ri.cpu().numpy(), np.repeat(np.arange(lens.size), lens)[order])
+    assert np.array_equal(perm.cpu().numpy(), order)
+    A.sync_status()
