@@ -41,3 +41,21 @@ def test_rows_bit_exact(oracle, K):
         want = ref.copy()
         want[[0, 5, 100, 101]] = 0.0
         assert np.array_equal(bits(out), bits(want))
+
+
+@pytest.mark.parametrize("K", [4, 16, 32, 128])
+def test_mostly_empty_rows(oracle, K):
+    """Runs of empty rows about as long as a group walks before it searches, and far longer."""
+    lens = np.concatenate([([0] * gap + [n]) for gap in (0, 1, 15, 16, 17, 18, 33, 3000)
+                           for n in (1, 2, 5)] + [[0] * 40])
+    rp = np.zeros(lens.size + 1, np.int32)
+    np.cumsum(lens, out=rp[1:])
+    rng = np.random.default_rng(K)
+    ci = np.concatenate([np.sort(rng.choice(90, n, replace=False)) for n in lens]).astype(np.int32)
+    a = S.CSR(rp, ci, rng.uniform(0.5, 1.5, ci.size).astype(np.float32), lens.size, 90)
+    assert a.n_rows > 4 * a.nnz
+    X, Y = S.dense_normal((a.n_rows, K), 1), S.dense_normal((90, K), 2)
+    rpd, cid, av = csr_dev(a)
+    out = A.sddmm(rpd, cid, to_dev(X), to_dev(Y), aval=av)
+    assert np.array_equal(bits(out), bits(oracle.sddmm_f32_group(a.rowptr, a.colind, X, Y, aval=a.val)))
+    A.sync_status()
