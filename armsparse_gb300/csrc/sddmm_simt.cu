@@ -218,11 +218,14 @@ sddmm_rows(int M, int N, int K, int nnz, int CH, const int *__restrict__ rowptr,
         for (int u = 0; u < 4; ++u)
             if (g + u * G < nq) v[u] = B::load_here(row + 4 * (g + u * G));
     };
-    auto column = [&](int e) { return e < e1 ? ld_stream(colind + e) : -1; };
+    // (unsigned: an entry ahead of 2^31 - 1 of them is past e1, not below zero)
+    auto column = [&](unsigned e) {
+        return e < static_cast<unsigned>(e1) ? ld_stream(colind + e) : -1;
+    };
     auto in_range = [&](int c) { return static_cast<unsigned>(c) < static_cast<unsigned>(N); };
     typename B::Raw x[4], y[4], yn[4];
     int held = -1;  // the row that x holds
-    int c = column(e0), cn = column(e0 + 1);
+    int c = column(e0), cn = column(e0 + 1u);
     if (in_range(c)) load(Y + c * ldy, y);
     for (int e = e0; e < e1; ++e) {  // every branch below is the same for the whole group
         while (e >= re && r + 1 < M) {
@@ -231,7 +234,7 @@ sddmm_rows(int M, int N, int K, int nnz, int CH, const int *__restrict__ rowptr,
             re = __ldg(rowptr + r + 1);
         }
         if (in_range(cn)) load(Y + cn * ldy, yn);
-        const int cnn = column(e + 2);
+        const int cnn = column(e + 2u);
         const bool row_ok = rs <= e && re > e;
         if (row_ok && in_range(c)) {
             if (held != r) {

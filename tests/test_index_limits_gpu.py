@@ -1,0 +1,33 @@
+"""Calls with as many entries as an int counts (2^31 - 1): the kernels read ahead of the entry they
+work on, and the last entries' look-ahead has to end at the last entry."""
+import pytest
+import torch
+
+import armsparse_gb300 as A
+from gpu_util import dev
+
+pytestmark = pytest.mark.gpu
+NNZ = 2 ** 31 - 1
+
+
+def _rowptr(*ends):
+    return torch.tensor([0, *ends], dtype=torch.int32, device=dev())
+
+
+def _columns():
+    """Column 1 for the last three entries, else 0."""
+    ci = torch.zeros(NNZ, dtype=torch.int32, device=dev())
+    ci[-3:] = 1
+    return ci
+
+
+def test_sddmm_reads_no_column_past_the_last():
+    X = torch.tensor([[1.0, 2, 3, 4], [0, 0, 0, 0], [2, 0, 1, 0]], device=dev())
+    Y = torch.tensor([[1.0, 1, 1, 1], [5, 0, 7, 0]], device=dev())
+    out = A.sddmm(_rowptr(5, 5, NNZ), _columns(), X, Y)
+    A.sync_status()
+    want = X @ Y.T
+    assert out[:5].tolist() == [want[0, 0].item()] * 5
+    assert out[-3:].tolist() == [want[2, 1].item()] * 3
+    for lo in range(5, NNZ - 3, 1 << 28):
+        assert bool((out[lo:min(lo + (1 << 28), NNZ - 3)] == want[2, 0]).all())
