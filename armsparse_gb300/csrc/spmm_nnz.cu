@@ -148,8 +148,8 @@ spmm_nnzsplit(int M, int K, int N, int nnz, int CH, const int *__restrict__ rowp
     if (e0l >= nnz) return;
     const int e0 = static_cast<int>(e0l);
     // entries past the last row's end (a row pointer that stops short of nnz) belong to no row
-    const int e1 = static_cast<int>(
-        min(min(e0l + CH, static_cast<long>(nnz)), static_cast<long>(__ldg(rowptr + M))));
+    const int e1 = static_cast<int>(max(
+        0L, min(min(e0l + CH, static_cast<long>(nnz)), static_cast<long>(__ldg(rowptr + M)))));
     const int tile0 = blockIdx.y * TILE;
     auto count = [&](bool p) { return __popc(__ballot_sync(gmask, p) & gmask); };
     const char *bcol[CPL];  // this lane's columns of row 0 of B (column 0 for a lane past N)
@@ -176,17 +176,18 @@ spmm_nnzsplit(int M, int K, int N, int nnz, int CH, const int *__restrict__ rowp
         return count(g > 0 ? w < below : w <= e) == 0;
     };
     using Val = decltype(lane_val(T()));
-    auto load_entry = [&](int e, int &k, Val &v) {
+    // (unsigned: an entry ahead of 2^31 - 1 of them is past e1, not below zero)
+    auto load_entry = [&](unsigned e, int &k, Val &v) {
         k = -1;
         v = 0;
-        if (e < e1) {
+        if (e < static_cast<unsigned>(e1)) {
             k = ld_stream(colind + e);
             v = lane_val(ld_stream(val + e));
         }
     };
     int re = ends(r0), k, base = e0;
     Val v;
-    load_entry(base + g, k, v);
+    load_entry(static_cast<unsigned>(base) + g, k, v);
     bool good = e0 < e1 && rs0 >= 0 && rs0 <= e0 && sound(re, e0);
     if (e0 < e1 && !good) flag(status, kFlagBadRowptr);
     int row = r0;                      // the row that the running sums belong to
@@ -251,7 +252,7 @@ spmm_nnzsplit(int M, int K, int N, int nnz, int CH, const int *__restrict__ rowp
         // the next batch's entries and window, in flight meanwhile
         int kn, rn = r0 + count(re <= next), ren = ends(rn);
         Val vn;
-        load_entry(next + g, kn, vn);
+        load_entry(static_cast<unsigned>(next) + g, kn, vn);
         if (g >= cnt) {
             k = -1;
         } else if (static_cast<unsigned>(k) >= static_cast<unsigned>(K)) {
@@ -428,11 +429,12 @@ spmm_nnzme(int M, int K, int N, int nnz, int CH, const int *__restrict__ rowptr,
         float acc[E];
 #pragma unroll
         for (int i = 0; i < E; ++i) acc[i] = 0.0f;
-        for (int base = e; base < se; base += 32) {
-            const int ee = base + lane;
+        const unsigned last = static_cast<unsigned>(se);  // unsigned: entries ahead of it stay above
+        for (unsigned base = e; base < last; base += 32) {
+            const unsigned ee = base + lane;
             int k = -1;
             float v = 0.0f;
-            if (ee < se) {
+            if (ee < last) {
                 k = ld_stream(colind + ee);
                 v = to_f32(ld_stream(val + ee));
                 if (static_cast<unsigned>(k) >= static_cast<unsigned>(K)) {
@@ -440,7 +442,7 @@ spmm_nnzme(int M, int K, int N, int nnz, int CH, const int *__restrict__ rowptr,
                     k = -1;
                 }
             }
-            const int cnt = min(32, se - base);
+            const int cnt = static_cast<int>(min(32u, last - base));
             for (int t = 0; t < cnt; t += S * U) {  // sub-group sg: entries t + sg + S*u
                 int kk[U];
                 float vv[U];
@@ -474,7 +476,7 @@ spmm_nnzme(int M, int K, int N, int nnz, int CH, const int *__restrict__ rowptr,
 #pragma unroll
                                 for (int i = 0; i < E; ++i) d[u] = fmaf(b[u][i], V::at(fr, i), d[u]);
                         }
-                        write_dots_me<U, GROUP>(d, kk, gmask, g, base + t + sg, S, nnz, perm, dA,
+                        write_dots_me<U, GROUP>(d, kk, gmask, g, static_cast<int>(base) + t + sg, S, nnz, perm, dA,
                                                 status);
                     }
                 } else {
@@ -497,7 +499,7 @@ spmm_nnzme(int M, int K, int N, int nnz, int CH, const int *__restrict__ rowptr,
                             d[u] = 0.0f;
                             if (col_ok) V::dot(b[u], fr, d[u]);
                         }
-                        write_dots_me<U, GROUP>(d, kk, gmask, g, base + t + sg, S, nnz, perm, dA,
+                        write_dots_me<U, GROUP>(d, kk, gmask, g, static_cast<int>(base) + t + sg, S, nnz, perm, dA,
                                                 status);
                     }
                 }

@@ -31,3 +31,21 @@ def test_sddmm_reads_no_column_past_the_last():
     assert out[-3:].tolist() == [want[2, 1].item()] * 3
     for lo in range(5, NNZ - 3, 1 << 28):
         assert bool((out[lo:min(lo + (1 << 28), NNZ - 3)] == want[2, 0]).all())
+
+
+@pytest.mark.parametrize("name", ["nnzsplit_v4_g32_c1_ch1024", "nnzsplit_v16_g8_c1_ch128",
+                                  "nnzme_v16_g8_ch1024"])
+def test_entry_balanced_reads_no_entry_past_the_last(name):
+    variant = A.spmm_variants(torch.bfloat16).index(name) + 1
+    rp, ci = _rowptr(5, NNZ - 3, NNZ), _columns()  # the last row: three entries of column 1
+    v = torch.ones(NNZ, dtype=torch.bfloat16, device=dev())
+    B = torch.zeros(2, 8, dtype=torch.bfloat16, device=dev())
+    B[1] = torch.arange(8)
+    C = A.spmm(rp, ci, v, B, variant=variant)
+    A.sync_status()
+    assert C.tolist() == [[0.0] * 8, [0.0] * 8, [3.0 * i for i in range(8)]]
+    F = torch.ones(3, 8, dtype=torch.bfloat16, device=dev())
+    C, dA = A.spmm_sddmm(rp, ci, v, B, F, variant=variant)
+    A.sync_status()
+    assert C[2].tolist() == [3.0 * i for i in range(8)]
+    assert dA[:5].tolist() == [0.0] * 5 and dA[-4:].tolist() == [0.0, 28.0, 28.0, 28.0]
