@@ -32,7 +32,7 @@ constexpr int kBatch = 4;       // rows of B loaded together
 // The first 64 entries of kBatch rows of B, two per lane.
 struct Batch {
     float a[kBatch];
-    int s[kBatch], e[kBatch];        // the rows' extents (empty past the end)
+    unsigned s[kBatch], e[kBatch];   // the rows' extents (empty past the end)
     int j[kBatch][2];
     float b[kBatch][2];
 };
@@ -65,26 +65,29 @@ spgemm_dense(int M, int K, int N, int tile, int nnz_a, int nnz_b, const int *__r
 
     int lo, hi;
     row_range(rp1, static_cast<int>(row), nnz_a, status, lo, hi);
-    for (int base = lo; base < hi; base += 32) {
+    // entries are counted unsigned: one read ahead of 2^31 - 1 of them is past the end, not below zero
+    const unsigned a_end = hi;
+    for (unsigned base = lo; base < a_end; base += 32) {
         // this lane's A entry: its value and the extent of B's row
-        const int e = base + lane;
+        const unsigned e = base + lane;
         float a = 0.0f;
-        int bs = 0, be = 0;
-        if (e < hi) {
+        unsigned bs = 0, be = 0;
+        if (e < a_end) {
             const int k = ld_stream(ci1 + e);
             a = ld_stream(v1 + e);
             if (static_cast<unsigned>(k) >= static_cast<unsigned>(K)) {
                 flag(status, kFlagBadColind);
             } else {
-                bs = __ldg(rp2 + k);
-                be = __ldg(rp2 + k + 1);
-                if (bs < 0 || be < bs || be > nnz_b) {
+                const int s = __ldg(rp2 + k), t = __ldg(rp2 + k + 1);
+                if (s < 0 || t < s || t > nnz_b) {
                     flag(status, kFlagBadRowptr);
-                    bs = be = 0;
+                } else {
+                    bs = s;
+                    be = t;
                 }
             }
         }
-        const int cnt = min(32, hi - base);
+        const int cnt = static_cast<int>(min(32u, a_end - base));
         auto load = [&](int u0, Batch &x) {
 #pragma unroll
             for (int q = 0; q < kBatch; ++q) {
@@ -95,7 +98,7 @@ spgemm_dense(int M, int K, int N, int tile, int nnz_a, int nnz_b, const int *__r
                 if (u0 + q >= cnt) x.e[q] = x.s[q];  // past A's entries: nothing to apply
 #pragma unroll
                 for (int h = 0; h < 2; ++h) {
-                    const int t = x.s[q] + 32 * h + lane;
+                    const unsigned t = x.s[q] + 32 * h + lane;
                     x.j[q][h] = -1;
                     x.b[q][h] = 0.0f;
                     if (t < x.e[q]) {
@@ -122,11 +125,11 @@ spgemm_dense(int M, int K, int N, int tile, int nnz_a, int nnz_b, const int *__r
             load(u0 + kBatch, next);
 #pragma unroll
             for (int q = 0; q < kBatch; ++q) {
-                const int n = x.e[q] - x.s[q];
+                const int n = static_cast<int>(x.e[q] - x.s[q]);
                 apply(x.a[q], lane < n, x.j[q][0], x.b[q][0]);
                 if (n > 32) apply(x.a[q], 32 + lane < n, x.j[q][1], x.b[q][1]);
-                for (int t0 = x.s[q] + 64; t0 < x.e[q]; t0 += 32) {  // longer rows of B
-                    const int t = t0 + lane;
+                for (unsigned t0 = x.s[q] + 64; t0 < x.e[q]; t0 += 32) {  // longer rows of B
+                    const unsigned t = t0 + lane;
                     const bool has = t < x.e[q];
                     apply(x.a[q], has, has ? __ldg(ci2 + t) : 0, has ? __ldg(v2 + t) : 0.0f);
                 }

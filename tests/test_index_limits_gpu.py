@@ -49,3 +49,18 @@ def test_entry_balanced_reads_no_entry_past_the_last(name):
     A.sync_status()
     assert C[2].tolist() == [3.0 * i for i in range(8)]
     assert dA[:5].tolist() == [0.0] * 5 and dA[-4:].tolist() == [0.0, 28.0, 28.0, 28.0]
+
+
+@pytest.mark.parametrize("length", [70, 2, 33])  # of B's last row, one past whole steps of 32
+def test_spgemm_reads_no_entry_past_the_last(length):
+    b_rp = _rowptr(NNZ - length, NNZ)
+    b_ci = torch.zeros(NNZ, dtype=torch.int32, device=dev())
+    b_ci[-length:] = torch.arange(length, dtype=torch.int32, device=dev())
+    b_v = torch.ones(NNZ, device=dev())
+    a_rp = _rowptr(1, 2)
+    a_ci = torch.tensor([1, 1], dtype=torch.int32, device=dev())
+    a_v = torch.tensor([2.0, 3.0], device=dev())
+    C = A.spgemm_dense(a_rp, a_ci, a_v, b_rp, b_ci, b_v, 80)
+    A.sync_status()
+    rest = [0.0] * (80 - length)
+    assert C.tolist() == [[2.0] * length + rest, [3.0] * length + rest]
