@@ -45,19 +45,17 @@ __device__ __forceinline__ uint16_t f32_to_bf16(float f) {
 // A ReLU applied at an output store when `relu` is set (negative -> 0; -0 and NaN pass).
 __device__ __forceinline__ float relu_if(float v, bool relu) { return relu && v < 0.0f ? 0.0f : v; }
 
-// Long rows are left by the row kernels to the long-row kernel (spmm_long.cu); rows with more
-// than kHugeRow entries are listed from the end of its list, which it takes first.
+// Rows with more than kLongRow entries are left by the row kernels to the long-row kernel
+// (spmm_long.cu); rows with more than kHugeRow are listed from the end of its list, which it
+// takes first. The long-row kernel keeps a row's chain fed but runs fewer chains at once than the
+// row kernels, so it pays for rows that would outlast the rest of the grid, not for shorter ones
+// that are many. Four times the mean (64 at least) in place of 256 gained where such rows are few
+// (19,717 rows of mean 5 at width 47: 47.5 -> 32.5 us; 300,000 power-law rows at width 128:
+// 1026 -> 962) and lost more where they hold much of the matrix, which the sizes of a call do
+// not tell: 100,000 rows of which a fifth hold 205 entries and the others none, 165 -> 442 us at
+// width 128; a tenth of 100 beside rows of 5, 83 -> 197; exponential lengths of mean 25, 115 -> 129.
+constexpr int kLongRow = 256;
 constexpr int kHugeRow = 16384;
-// A row is long past four times the mean, between 64 and 256 entries: in a matrix of short rows
-// the few longer ones are the row kernels' critical path (a group walks its row a few entries
-// per memory latency), where the long-row kernel has a whole row's loads in flight; in a matrix
-// whose rows are all alike, none is listed. Measured at 256 and 64: an aggregation of 19,717
-// rows (mean 5) at width 47 47.5 and 32.5 us, 300,000 power-law rows (mean 19) at width 128
-// 1026 and 962 us; 4096 rows of mean 41 stay on the row kernel either way.
-inline int long_row_threshold(long long nnz, long long rows) {
-    const long long t = rows > 0 ? 4 * ((nnz + rows - 1) / rows) : 0;
-    return static_cast<int>(t < 64 ? 64 : t > 256 ? 256 : t);
-}
 
 // Lists row `row` (of `len` entries) for the long-row kernel: counters [0] rows listed from the
 // front, [2] huge rows listed from the end of the M-entry list.

@@ -9,8 +9,9 @@
 //   in CSR order and updates its accumulators with fmaf(b, v, acc). Each output element is
 //   therefore exactly the reference's fused-FMA chain. Blocks are 256 threads; blockIdx.x
 //   runs over row blocks and blockIdx.y over column tiles, so the CTAs resident at any
-//   moment share one column tile of B, which stays in L2. Long rows (long_row_threshold) are
-//   skipped here and computed by the long-row kernel (spmm_long.cu), which keeps the same chains.
+//   moment share one column tile of B, which stays in L2. Rows with more than kLongRow
+//   entries are skipped here and computed by the long-row kernel (spmm_long.cu), which keeps the
+//   same chains.
 #include <limits.h>
 #include <stdio.h>
 
@@ -476,11 +477,10 @@ as_status spmm_launch(as_ctx *ctx, int dtype, int variant, const SpmmArgs &a, cu
         return fail(AS_ERR_UNSUPPORTED, "spmm: N too large for this variant's column tile");
     // long rows go to the long-row kernel (a matrix of fewer entries than one has none)
     LongRows lr{INT_MAX, nullptr, ctx->d_long};
-    const int thresh = long_row_threshold(a.nnz, a.M);
-    if (a.nnz > thresh && a.M > 0) {
+    if (a.nnz > kLongRow && a.M > 0) {
         as_status st = scratch_list(ctx, a.M, s, &lr.list);
         if (st != AS_OK) return st;
-        if (lr.list) lr.thresh = thresh;
+        if (lr.list) lr.thresh = kLongRow;
     }
     bool ok = false;
     if (v.pf) {

@@ -10,7 +10,7 @@
 // in CSR order, so an empty row stays at -10000.
 //
 // One warp per row; each lane owns CPL vectors of E columns of the row's column tile (16-byte
-// loads where the layout allows, scalar otherwise). Long rows (long_row_threshold) are left to the long-row kernel (spmm_long.cu,
+// loads where the layout allows, scalar otherwise). Rows with more than kLongRow entries are left to the long-row kernel (spmm_long.cu,
 // launched next with the same reduction as its chain step), as in the row-split SpMM: a hub
 // row would otherwise keep one warp busy for the whole call.
 #include <limits.h>
@@ -142,11 +142,10 @@ as_status spmm_reduce_launch(as_ctx *ctx, int op, const SpmmArgs &a, cudaStream_
     // long rows go to the long-row kernel
     int thresh = INT_MAX;
     int *list = nullptr;
-    const int long_row = long_row_threshold(a.nnz, a.M);
-    if (a.nnz > long_row && a.M > 0) {
+    if (a.nnz > kLongRow && a.M > 0) {
         as_status st = scratch_list(ctx, a.M, s, &list);
         if (st != AS_OK) return st;
-        if (list) thresh = long_row;
+        if (list) thresh = kLongRow;
     }
     const bool vec = a.N % 4 == 0 && a.ldb % 4 == 0 && a.ldc % 4 == 0 &&
                      reinterpret_cast<uintptr_t>(a.B) % 16 == 0 &&

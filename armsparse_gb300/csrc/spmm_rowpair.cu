@@ -19,7 +19,7 @@
 // is ignored (the entry counts for its own row), and a flagged first entry of a segment reuses
 // a zero segment. A column index out of range is flagged and its entry skipped.
 //
-// Long pairs (long_row_threshold) are left to the long-row kernel (spmm_long.cu, its
+// Pairs with more than kLongRow entries are left to the long-row kernel (spmm_long.cu, its
 // row-pair step): a unit per row of the pair runs the same chain over the entries it includes,
 // each with its own column's B segment (identical to the reused one in a well-formed layout).
 #include <limits.h>
@@ -169,11 +169,10 @@ as_status spmm_rowpair_launch(as_ctx *ctx, const SpmmArgs &a, const uint8_t *fla
     // long pairs go to the long-row kernel
     int thresh = INT_MAX;
     int *list = nullptr;
-    const int long_pair = long_row_threshold(a.nnz, (static_cast<long>(a.M) + 1) / 2);
-    if (a.nnz > long_pair && a.M > 0) {
+    if (a.nnz > kLongRow && a.M > 0) {
         as_status st = scratch_list(ctx, a.M, s, &list);
         if (st != AS_OK) return st;
-        if (list) thresh = long_pair;
+        if (list) thresh = kLongRow;
     }
     // widest vectors the layout allows: float4 x 2 for wide B, float2, then scalars
     if (wide)

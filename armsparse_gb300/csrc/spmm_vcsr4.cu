@@ -8,7 +8,7 @@
 // skipped (the layout cannot tell a stored zero from an empty slot), so every output is one
 // fused chain over the row's nonzero entries in column order: bit for bit the CSR SpMM of the
 // same matrix without stored zeros. The four rows of a block are adjacent in B, which the
-// gathers see as one run of 4 * ldb elements. Long rows (long_row_threshold) are left to
+// gathers see as one run of 4 * ldb elements. Rows with more than kLongRow slots are left to
 // the long-row kernel (spmm_long.cu, its zero-skipping step), as in the row-split SpMM.
 #include <limits.h>
 
@@ -120,11 +120,10 @@ as_status spmm_vcsr4_launch(as_ctx *ctx, int M, int K, int N, int nslots, const 
         return fail(AS_ERR_UNSUPPORTED, "spmm vcsr4: N too large");
     // long rows go to the long-row kernel
     LongList lr{INT_MAX, nullptr, ctx->d_long};
-    const int long_row = long_row_threshold(nslots, M);
-    if (nslots > long_row && M > 0) {
+    if (nslots > kLongRow && M > 0) {
         as_status st = scratch_list(ctx, M, s, &lr.list);
         if (st != AS_OK) return st;
-        if (lr.list) lr.thresh = long_row;
+        if (lr.list) lr.thresh = kLongRow;
     }
     if (wide)
         launch<16, 2>(M, K, N, nslots, vrowptr, vcolind, vval, B, ldb, C, ldc, beta, ctx->d_status, lr, s);
