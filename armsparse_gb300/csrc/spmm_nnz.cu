@@ -119,15 +119,29 @@ __device__ __forceinline__ const char *row_at(const char *p, int kk, unsigned ld
 __device__ __forceinline__ float lane_val(float v) { return v; }
 __device__ __forceinline__ unsigned lane_val(uint16_t v) { return v; }
 
-// CTAs per SM to leave registers for: the gathers live on warps in flight, so four (64
-// registers) wherever a step's loads and the running sums fit, else two. (Width 256 in bf16 on
-// 35.8M entries: 2.14 ms with 64 registers, 2.54 with 76; fused 3.5 ms with 64 and a few
-// spilled, 5.4 with 100.)
-template <int VB, int CPL, int U, int E>
-constexpr int ctas_per_sm() { return U * CPL * VB / 4 + CPL * E <= 24 ? 4 : 2; }
+// CTAs per SM to leave registers for. The gathers live on warps in flight, and a spill or a step
+// that waits for registers costs more than a CTA gives, so the line is measured per kind of kernel,
+// 2 to 6 CTAs each on four matrices (uniform rows of 3 and of 20, power-law rows of 4.2M and 16.8M
+// entries, widths 16 to 256); geometric means of the time against that of the row-by-row walk:
+// - four (64 registers) wherever a step's loads and the running sums are at most 24 registers: fp32
+//   float4 0.78 with four, 0.84 with three, 0.86 with five; fused bf16 of 256 columns 0.93 with four
+//   in spite of 88 bytes spilled, 1.10 with two, 1.02 with five;
+// - three (80 registers) where a lane holds two vectors and a step takes eight entries of narrow
+//   ones (0.68-0.71; 0.76-0.78 with four, which spilled 128-156 bytes; 0.76-0.80 with two), and for
+//   the fused fp32 float4 x 2 (0.75; 0.78 with two, 0.85 with four);
+// - else two: fp32 float4 x 2 0.81 (three 0.81, and a fifth slower on the smaller power-law matrix),
+//   bf16 of 512 columns 0.81 (three 0.81, four 0.99), eight entries of bf16 x 8 0.61 (three 0.65).
+// Uniform rows of 20 lose by the walk in some kernels whatever the count: scalar lanes x 2 in fp32
+// up to 1.28 (mean 0.90), eight entries of float4 by sixteens up to 1.24 (mean 0.73).
+template <int VB, int CPL, int U, int E, bool FUSE>
+constexpr int ctas_per_sm() {
+    constexpr int regs = U * CPL * VB / 4 + CPL * E;
+    if (CPL == 2 && (U == 8 ? regs <= 24 : FUSE && regs > 24 && regs <= 40)) return 3;
+    return regs <= 24 ? 4 : 2;
+}
 
 template <typename T, int VB, int GROUP, int CPL, int U, bool FUSE>
-__global__ void __launch_bounds__(kThreads, ctas_per_sm<VB, CPL, U, Vec<T, VB>::E>())
+__global__ void __launch_bounds__(kThreads, ctas_per_sm<VB, CPL, U, Vec<T, VB>::E, FUSE>())
 spmm_nnzsplit(int M, int K, int N, int nnz, int CH, const int *__restrict__ rowptr,
               const int *__restrict__ colind, const T *__restrict__ val,
               const T *__restrict__ B, long ldb, float *__restrict__ C, long ldc, float beta,
