@@ -57,8 +57,24 @@ __device__ __forceinline__ void load_c(const float *p, float *v) {
 
 constexpr int kThreads = 256;
 
+// Resident CTAs that a kernel's registers have to leave room for (1: as the compiler likes). The
+// prefetching kernels take four. Where a batch is one step (GROUP == U) the registers of the partial
+// step cost some kernels a CTA, and with it up to a fifth of their speed: those are held to what
+// they had without it (bf16, 2M entries in uniform rows of 20, width 256, 16-byte vectors by fours x 2:
+// 203 us with 83 registers, 158 with 80; 171 entry by entry).
 template <typename T, int VB, int GROUP, int CPL, int U, bool PF>
-__global__ void __launch_bounds__(kThreads, PF ? 4 : 1)
+constexpr int rowsplit_ctas() {
+    if (PF) return 4;
+    if (GROUP != U) return 1;
+    if (sizeof(T) == 4) return VB == 4 && CPL == 4 ? 5 : 1;
+    if (VB == 8 && U == 4 && CPL == 2) return 4;
+    return (VB == 16 && U == 4 && CPL == 2) || (VB == 2 && CPL == (U == 4 ? 4 : 2)) ||
+                   (VB == 4 && U == 8 && CPL == 2)
+               ? 3 : 1;
+}
+
+template <typename T, int VB, int GROUP, int CPL, int U, bool PF>
+__global__ void __launch_bounds__(kThreads, rowsplit_ctas<T, VB, GROUP, CPL, U, PF>())
 spmm_rowsplit(int M, int K, int N, int nnz, const int *__restrict__ rowptr,
               const int *__restrict__ colind, const T *__restrict__ val,
               const T *__restrict__ B, long ldb, float *__restrict__ C, long ldc, float beta,
@@ -194,9 +210,12 @@ spmm_rowsplit(int M, int K, int N, int nnz, const int *__restrict__ rowptr,
         };
         int t = 0;
         for (; t + U <= cnt; t += U) step(t, std::false_type());
-        if constexpr (GROUP >= U) {
+        // a batch that never fills a step goes entry by entry (a part step of 8 cost 55 us for 38),
+        // and so do the prefetching bf16 kernels of four vectors, whose 64 registers do not hold
+        // a part step too (2.0 times as long on rows of mean 3, 1.2 of mean 20)
+        if constexpr (GROUP >= U && !(PF && sizeof(T) == 2 && CPL == 4)) {
             if (t < cnt) step(t, std::true_type());
-        } else {  // a batch never fills a step: entry by entry (a part step of 8 cost 55 us for 38)
+        } else {
             for (; t < cnt; ++t) {
                 const int kk = __shfl_sync(gmask, k, t, GROUP);
                 const float vv = __shfl_sync(gmask, v, t, GROUP);
