@@ -87,6 +87,18 @@ __device__ __forceinline__ void row_range(const int *rowptr, int r, int nnz, uns
 template <int GROUP>
 __device__ __forceinline__ int find_row(const int *__restrict__ rowptr, int M, long e, int g,
                                         unsigned gmask) {
+    if constexpr (GROUP == 1) {  // no lanes to share it: plain halving, no ballots
+        int lo = 0, hi = M;
+#pragma unroll 1
+        while (hi - lo > 1) {
+            const int mid = lo + (hi - lo) / 2;
+            if (__ldg(rowptr + mid) <= e)
+                lo = mid;
+            else
+                hi = mid;
+        }
+        return lo;
+    }
     long lo = 0, hi = M;
     while (hi - lo > 1) {
         const long width = hi - lo;

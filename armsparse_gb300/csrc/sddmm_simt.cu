@@ -14,6 +14,8 @@
 // (acc += shfl_xor(acc, off), off = G/2 .. 1); lane 0 writes s_e * sum. bf16 operands use the
 // mixed-precision FMA of sm_100+ (a bf16 x bf16 product is exact in fp32), so the bf16 kernel
 // gives bit for bit the fp32 kernel's result on the widened values.
+#include <algorithm>
+
 #include "common.cuh"
 #include "internal.h"
 
@@ -21,7 +23,7 @@ namespace as {
 namespace {
 
 constexpr int kThreads = 256;
-constexpr int kWalkRows = 16;  // rows walked before the next one is searched for
+constexpr int kWalkRows = 64;  // rows walked (from L1) before the next one is searched for (from L2)
 
 // acc = fma(x0, y0, acc); acc = fma(x1, y1, acc) for the bf16 halves of x and y, in order.
 __device__ __forceinline__ void fma_bf16_seq2(unsigned x, unsigned y, float &acc) {
@@ -117,15 +119,17 @@ __device__ __forceinline__ float lane_chain(const T *xr, const T *yr, int K, int
 template <int G>
 __device__ __forceinline__ void next_row(const int *__restrict__ rowptr, int M, int e, int g,
                                          unsigned gmask, int &r, int &rs, int &re) {
-    for (int i = 0; e >= re && r + 1 < M; ++i) {
-        if (i == kWalkRows) {
-            r = find_row<G>(rowptr, M, e, g, gmask);
-            rs = __ldg(rowptr + r);
-            re = __ldg(rowptr + r + 1);
-            return;
-        }
+    if (e < re) return;
+    const int stop = r < M - kWalkRows ? r + kWalkRows : M - 1;
+#pragma unroll 1
+    while (e >= re && r < stop) {
         ++r;
         rs = re;
+        re = __ldg(rowptr + r + 1);
+    }
+    if (e >= re && r + 1 < M) {
+        r = find_row<G>(rowptr, M, e, g, gmask);
+        rs = __ldg(rowptr + r);
         re = __ldg(rowptr + r + 1);
     }
 }
@@ -281,9 +285,17 @@ as_status launch_group(as_ctx *ctx, int M, int N, int K, int nnz, const int *row
     // registers and 70 us of 353 at K = 128)
     const bool resident = !COO && vec && K > 0 && K <= 16 * G && N > 0 && M <= 4L * nnz;
     int CH = G >= 32 ? 4 : 128 / G;  // edges per group: more for short dot products
-    if (resident) {  // as many as leave two waves of full SMs, 4 to 64
-        const long all = static_cast<long>(nnz) * G / (2L * 2048 * ctx->sms);
-        CH = static_cast<int>(all < 4 ? 4 : all > 64 ? 64 : all);
+    if (resident) {
+        // Edges per group: as many as leave four waves of the CTAs that an SM holds (four of fp32, five
+        // of bf16), up to 64; where that is under 16, as many as leave two whole waves, up to 16: a
+        // chunk's first row is searched for, which a few short edges do not pay for (2.4M entries, K =
+        // 20: 99 us with chunks of 7, 72 with 16; 600,000, K = 128: 41 and 35), but a chunk is walked
+        // in order (20,000 entries, K = 132: 8 us with chunks of 4, 12 with 16).
+        const long lanes = static_cast<long>(nnz) * G;
+        const long wave = (sizeof(T) == 4 ? 4L : 5L) * kThreads * ctx->sms;
+        long n = lanes / (4L * 4 * kThreads * ctx->sms);
+        if (n < 16) n = std::min(16L, static_cast<long>(ceil_div(lanes, 2 * wave)));
+        CH = static_cast<int>(n < 4 ? 4 : n > 64 ? 64 : n);
     }
     const long groups = ceil_div(nnz, CH);
     const unsigned grid = static_cast<unsigned>(ceil_div(groups * G, kThreads));
