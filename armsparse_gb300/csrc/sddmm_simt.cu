@@ -24,6 +24,7 @@ namespace {
 
 constexpr int kThreads = 256;
 constexpr int kWalkRows = 64;  // rows walked (from L1) before the next one is searched for (from L2)
+constexpr int kFarRows = 16;   // rows an edge past which a chunk of sddmm_rows searches
 
 // acc = fma(x0, y0, acc); acc = fma(x1, y1, acc) for the bf16 halves of x and y, in order.
 __device__ __forceinline__ void fma_bf16_seq2(unsigned x, unsigned y, float &acc) {
@@ -134,23 +135,19 @@ __device__ __forceinline__ void next_row(const int *__restrict__ rowptr, int M, 
     }
 }
 
-// COO: rows come per edge from `rows` (any order); CSR: `rows` is the row pointer.
+// One group's edges e0 .. e1 - 1, one at a time. COO: rows come per edge from `rows` (any order);
+// CSR: `rows` is the row pointer and r the row of edge e0.
 template <typename T, bool VEC, int G, bool COO>
-__global__ void __launch_bounds__(kThreads)
-sddmm_group(int M, int N, int K, int nnz, int CH, const int *__restrict__ rows,
-            const int *__restrict__ colind, const float *__restrict__ aval,
-            const T *__restrict__ X, long ldx, const T *__restrict__ Y, long ldy,
-            float *__restrict__ out, unsigned *status) {
-    const long grp = (static_cast<long>(blockIdx.x) * kThreads + threadIdx.x) / G;
-    const int g = threadIdx.x % G;
-    const unsigned gmask =
-        G == 32 ? 0xffffffffu : (((1u << G) - 1u) << ((threadIdx.x & 31) & ~(G - 1)));
-    const long e0 = grp * CH;
-    if (e0 >= nnz) return;  // the whole group leaves together
-    const long e1 = e0 + CH < nnz ? e0 + CH : nnz;
-    int r = 0, rs = 0, re = 0;
+__device__ __forceinline__ void group_edges(int M, int N, int K, long e0, long e1, int r,
+                                            const int *__restrict__ rows,
+                                            const int *__restrict__ colind,
+                                            const float *__restrict__ aval,
+                                            const T *__restrict__ X, long ldx,
+                                            const T *__restrict__ Y, long ldy,
+                                            float *__restrict__ out, int g, unsigned gmask,
+                                            unsigned *status) {
+    int rs = 0, re = 0;
     if (!COO) {
-        r = find_row<G>(rows, M, e0, g, gmask);
         rs = __ldg(rows + r);
         re = __ldg(rows + r + 1);
     }
@@ -192,16 +189,35 @@ sddmm_group(int M, int N, int K, int nnz, int CH, const int *__restrict__ rows,
     }
 }
 
+template <typename T, bool VEC, int G, bool COO>
+__global__ void __launch_bounds__(kThreads)
+sddmm_group(int M, int N, int K, int nnz, int CH, const int *__restrict__ rows,
+            const int *__restrict__ colind, const float *__restrict__ aval,
+            const T *__restrict__ X, long ldx, const T *__restrict__ Y, long ldy,
+            float *__restrict__ out, unsigned *status) {
+    const long grp = (static_cast<long>(blockIdx.x) * kThreads + threadIdx.x) / G;
+    const int g = threadIdx.x % G;
+    const unsigned gmask =
+        G == 32 ? 0xffffffffu : (((1u << G) - 1u) << ((threadIdx.x & 31) & ~(G - 1)));
+    const long e0 = grp * CH;
+    if (e0 >= nnz) return;  // the whole group leaves together
+    const long e1 = e0 + CH < nnz ? e0 + CH : nnz;
+    const int r = COO ? 0 : find_row<G>(rows, M, e0, g, gmask);
+    group_edges<T, VEC, G, COO>(M, N, K, e0, e1, r, rows, colind, aval, X, ldx, Y, ldy, out, g,
+                                gmask, status);
+}
+
 // The CSR form where a lane's part of a row is at most four blocks (K <= 16 G) and rows are
 // aligned: X's row stays in registers while the row lasts, the next edge's Y row is loaded (and
 // the column of the one after it read) while the present edge is summed. The sums are
 // sddmm_group's, in the same order. What bounds it is Y's gathers, so warps in flight count: on a
-// graph of 6M entries with K = 128 it takes 354 us with four CTAs per SM (64 registers), 425 with
-// three, 655 with five (spills); two edges per turn, 488; sddmm_group 461. (K = 512: 1.24 and 2.23
+// graph of 6M entries with K = 128 it takes 350 us with four CTAs per SM (64 registers), 425 with
+// three, 655 with five (spills); two edges per turn, 488; sddmm_group 461; with the search in the
+// walk 423. bf16 rows leave room for five. (K = 512: 1.24 and 2.23
 // ms; K = 16: 0.21 and 0.31.) The loads are volatile because left to the compiler they move down
 // to their uses.
 template <typename T, int G>
-__global__ void __launch_bounds__(kThreads, 4)
+__global__ void __launch_bounds__(kThreads, sizeof(T) == 4 ? 4 : 5)
 sddmm_rows(int M, int N, int K, int nnz, int CH, const int *__restrict__ rowptr,
            const int *__restrict__ colind, const float *__restrict__ aval,
            const T *__restrict__ X, long ldx, const T *__restrict__ Y, long ldy,
@@ -216,7 +232,10 @@ sddmm_rows(int M, int N, int K, int nnz, int CH, const int *__restrict__ rowptr,
     const int e1 = CH < nnz - e0 ? e0 + CH : nnz;
     const int nq = K >> 2;
     int r = find_row<G>(rowptr, M, e0, g, gmask);
-    int rs = __ldg(rowptr + r), re = __ldg(rowptr + r + 1);
+    const long far = static_cast<long>(r) + kFarRows * CH;
+    const int far_start = far < M ? __ldg(rowptr + far) : e1;  // (read early, looked at late)
+    const int rs = __ldg(rowptr + r);
+    int re = __ldg(rowptr + r + 1);
     auto load = [&](const T *row, typename B::Raw (&v)[4]) {
 #pragma unroll
         for (int u = 0; u < 4; ++u)
@@ -231,15 +250,22 @@ sddmm_rows(int M, int N, int K, int nnz, int CH, const int *__restrict__ rowptr,
     int held = -1;  // the row that x holds
     int c = column(e0), cn = column(e0 + 1u);
     if (in_range(c)) load(Y + c * ldy, y);
+    // a chunk over more than kFarRows rows an edge (a long run of empty ones) goes the way that
+    // searches: the walk below is row by row, and a search in it costs it registers (so does one
+    // whose first row starts past its first edge: a malformed pointer)
+    if (far_start < e1 || rs > e0) {
+        group_edges<T, true, G, false>(M, N, K, e0, e1, r, rowptr, colind, aval, X, ldx, Y, ldy, out,
+                                       g, gmask, status);
+        return;
+    }
     for (int e = e0; e < e1; ++e) {  // every branch below is the same for the whole group
         while (e >= re && r + 1 < M) {
             ++r;
-            rs = re;
             re = __ldg(rowptr + r + 1);
         }
         if (in_range(cn)) load(Y + cn * ldy, yn);
         const int cnn = column(e + 2u);
-        const bool row_ok = rs <= e && re > e;
+        const bool row_ok = re > e;
         if (row_ok && in_range(c)) {
             if (held != r) {
                 load(X + r * ldx, x);
@@ -281,8 +307,7 @@ as_status launch_group(as_ctx *ctx, int M, int N, int K, int nnz, const int *row
                      reinterpret_cast<uintptr_t>(Y) % (4 * esz) == 0;
     const int G = group_size(K);
     // K in (0, 16 G]: every lane's blocks fit its registers
-    // (and rows are not mostly empty: its walk over them is row by row, the search costs it
-    // registers and 70 us of 353 at K = 128)
+    // (and rows are not mostly empty: most of its chunks would leave for the loop that searches)
     const bool resident = !COO && vec && K > 0 && K <= 16 * G && N > 0 && M <= 4L * nnz;
     int CH = G >= 32 ? 4 : 128 / G;  // edges per group: more for short dot products
     if (resident) {
