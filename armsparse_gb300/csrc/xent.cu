@@ -10,12 +10,12 @@
 // Backward: G[i, j] = (exp(x_j - lse_i) - [j == label]) * gscale / n in bf16 (round to nearest
 // even), zero in the padding columns C .. width-1; gscale is read from device memory (the
 // upstream gradient), so nothing synchronises. A thread works on its own row; its 16-byte loads
-// and stores each touch 32 rows per instruction of its warp, which evicts lines before they are
-// used whole. So a CTA moves its rows as one run between memory and shared memory, neighbouring
-// threads neighbouring pieces (a piece of padding per row keeps the accesses free of bank
-// conflicts), and the gradients take the scores' place there: 2.4M rows of 48 in 142 us, 253
-// without; with only the gradients parked 278. (The forward, with nothing to store, lost by it:
-// 106 us in place of 82.)
+// and stores each touch 32 rows per instruction of its warp. Where scores and gradients pass through
+// the caches without staying (park_rows), lines are evicted before they are used whole; there a CTA
+// moves its rows as one run between memory and shared memory, neighbouring threads neighbouring
+// pieces (a piece of padding per row keeps the accesses free of bank conflicts), and the gradients
+// take the scores' place there: 2.4M rows of 48 in 138 us, 253 without; with only the gradients
+// parked 278. (The forward, with nothing to store, lost by it: 106 us in place of 82.)
 #include "common.cuh"
 #include "internal.h"
 #include "spmm_vec.cuh"
@@ -111,18 +111,19 @@ xent_finish(int nparts, const float *__restrict__ partial, float inv_n, float *_
     if (threadIdx.x == 0) *loss = t * inv_n;
 }
 
-// VEC: 16-byte score loads and 16-byte gradient stores (width a multiple of 8, rows aligned).
-template <bool VEC>
+// VEC: 16-byte score loads and 16-byte gradient stores (width a multiple of 8, rows aligned). PARK
+// (with VEC): by way of shared memory.
+template <bool VEC, bool PARK>
 __global__ void __launch_bounds__(kThreads)
 xent_bwd(int n, int C, const uint16_t *__restrict__ S, long lds,
          const int64_t *__restrict__ labels, const float *__restrict__ lse_in,
          const float *__restrict__ gscale, float inv_n, uint16_t *__restrict__ G, long ldg,
          int width) {
     constexpr int kPitch = kMaxC / 8 + 1;  // 16-byte pieces per parked row
-    __shared__ uint4 parked[VEC ? kThreads * kPitch : 1];
+    __shared__ uint4 parked[PARK ? kThreads * kPitch : 1];
     const long row0 = static_cast<long>(blockIdx.x) * kThreads;
     const int rows = static_cast<int>(min(static_cast<long>(kThreads), n - row0));
-    if (VEC) {
+    if (PARK) {
         const int pieces = (C + 7) / 8;
         for (int j = threadIdx.x; j < rows * pieces; j += kThreads) {
             const int r = j / pieces, p = j - r * pieces;
@@ -133,7 +134,7 @@ xent_bwd(int n, int C, const uint16_t *__restrict__ S, long lds,
     } else if (threadIdx.x >= rows) {
         return;
     }
-    uint4 *mine = parked + (VEC ? threadIdx.x * kPitch : 0);
+    uint4 *mine = parked + (PARK ? threadIdx.x * kPitch : 0);
     const long i = row0 + min(static_cast<int>(threadIdx.x), rows - 1);  // past the end: not stored
     const uint16_t *row = S + i * lds;
     const int64_t t = labels[i];
@@ -146,10 +147,10 @@ xent_bwd(int n, int C, const uint16_t *__restrict__ S, long lds,
         if (8 * v >= width) break;
         float x[8], g[8];
         if (8 * v < C) {
-            if constexpr (VEC)
+            if constexpr (PARK)
                 unpack8(mine[v], x);
             else
-                load8<false>(row, v, C, x);
+                load8<VEC>(row, v, C, x);
         } else {
 #pragma unroll
             for (int q = 0; q < 8; ++q) x[q] = -INFINITY;
@@ -160,16 +161,16 @@ xent_bwd(int n, int C, const uint16_t *__restrict__ S, long lds,
             g[q] = (ok && j < C) ? (expf(x[q] - lse) - (j == t ? 1.0f : 0.0f)) * scale : 0.0f;
         }
         if (VEC) {
-            mine[v] =
-                make_uint4(pack_bf16x2(g[0], g[1]), pack_bf16x2(g[2], g[3]),
-                           pack_bf16x2(g[4], g[5]), pack_bf16x2(g[6], g[7]));
+            uint4 *dst = PARK ? mine + v : reinterpret_cast<uint4 *>(grow) + v;
+            *dst = make_uint4(pack_bf16x2(g[0], g[1]), pack_bf16x2(g[2], g[3]),
+                              pack_bf16x2(g[4], g[5]), pack_bf16x2(g[6], g[7]));
         } else {
 #pragma unroll
             for (int q = 0; q < 8; ++q)
                 if (8 * v + q < width) grow[8 * v + q] = f32_to_bf16(g[q]);
         }
     }
-    if (VEC) {
+    if (PARK) {
         __syncthreads();
         const int pieces = width / 8;
         for (int j = threadIdx.x; j < rows * pieces; j += kThreads) {
@@ -185,6 +186,17 @@ bool vec_rows(int C, long lds, const void *S, int width, long ldg, const void *G
     const bool s_ok = lds % 8 == 0 && lds >= Cv && reinterpret_cast<uintptr_t>(S) % 16 == 0;
     if (!G) return s_ok;
     return s_ok && width % 8 == 0 && ldg % 8 == 0 && reinterpret_cast<uintptr_t>(G) % 16 == 0;
+}
+
+// Whether the backward's rows go by way of shared memory, from 8 to 64 classes and up to 2.4M rows
+// timed both ways: rows of 32 classes or more whose scores and gradients together are past what L2
+// keeps (40 wide: 1M rows, 160 MB, 49 us and 53 parked, 2.4M rows 210 and 118; 48 wide: 400,000 rows
+// 25 and 27, 1M rows, 192 MB, 84 and 63; 32 wide: 2.4M rows 110 and 95), and for rows of a whole
+// line (over 56 classes) from 50 MB (64 wide: 200,000 rows 22.6 and 20.6, 400,000 rows 46 and 33).
+// Narrower rows use their lines whole soon enough (2.4M rows: 24 wide 75 and 88, 16 wide 43 and 64).
+bool park_rows(long n, int width, long lds, long ldg) {
+    const long bytes = 2 * n * (lds + ldg);
+    return width > 56 ? bytes > 50'000'000 : width >= 32 && bytes > 170'000'000;
 }
 
 }  // namespace
@@ -220,12 +232,10 @@ as_status xent_bwd_launch(as_ctx *ctx, int n, int C, const uint16_t *S, long lds
     if (n == 0) return AS_OK;
     const unsigned blocks = static_cast<unsigned>(ceil_div(n, kThreads));
     const float inv_n = 1.0f / static_cast<float>(n);
-    if (vec_rows(C, lds, S, width, ldg, G))
-        xent_bwd<true><<<blocks, kThreads, 0, s>>>(n, C, S, lds, labels, lse, gscale, inv_n, G,
-                                                   ldg, width);
-    else
-        xent_bwd<false><<<blocks, kThreads, 0, s>>>(n, C, S, lds, labels, lse, gscale, inv_n, G,
-                                                    ldg, width);
+    const auto kernel = !vec_rows(C, lds, S, width, ldg, G) ? xent_bwd<false, false>
+                        : park_rows(n, width, lds, ldg)     ? xent_bwd<true, true>
+                                                            : xent_bwd<true, false>;
+    kernel<<<blocks, kThreads, 0, s>>>(n, C, S, lds, labels, lse, gscale, inv_n, G, ldg, width);
     ctx->launches++;
     return check_cuda(cudaGetLastError(), "softmax xent backward launch");
 }
