@@ -92,16 +92,45 @@ scan_reduce(const int *__restrict__ in, long n, int *__restrict__ block_sums) {
     if (threadIdx.x == 0) block_sums[blockIdx.x] = total;
 }
 
-// Each CTA adds up the sums of the CTAs before it, then scans its own chunk.
+// One CTA: the exclusive scan of nb block sums in place, a chunk at a time.
+__global__ void __launch_bounds__(kThreads) scan_block_sums(int *sums, long nb) {
+    __shared__ int sw[kWarps];
+    int carry = 0;
+    for (long base = 0; base < nb; base += kScanChunk) {
+        const long first = base + static_cast<long>(threadIdx.x) * kScanItems;
+        int v[kScanItems];
+        int s = 0;
+#pragma unroll
+        for (int i = 0; i < kScanItems; ++i) {
+            v[i] = first + i < nb ? sums[first + i] : 0;
+            s += v[i];
+        }
+        int total;
+        int run = block_exclusive_scan(s, sw, total) + carry;
+#pragma unroll
+        for (int i = 0; i < kScanItems; ++i) {
+            if (first + i < nb) sums[first + i] = run;
+            run += v[i];
+        }
+        carry += total;
+    }
+}
+
+// Each CTA adds up the sums of the CTAs before it (`scanned`: finds the total in its own place),
+// then scans its own chunk.
 __global__ void __launch_bounds__(kThreads)
 scan_downsweep(const int *__restrict__ in, long n, const int *__restrict__ block_sums,
-               int *__restrict__ out, bool vec) {
+               int *__restrict__ out, bool vec, bool scanned) {
     __shared__ int sw[kWarps];
     const long base = static_cast<long>(blockIdx.x) * kScanChunk;
-    int before = 0;
-    for (int i = threadIdx.x; i < blockIdx.x; i += kThreads) before += block_sums[i];
     int prefix;
-    block_exclusive_scan(before, sw, prefix);
+    if (scanned) {
+        prefix = block_sums[blockIdx.x];
+    } else {
+        int before = 0;
+        for (unsigned i = threadIdx.x; i < blockIdx.x; i += kThreads) before += block_sums[i];
+        block_exclusive_scan(before, sw, prefix);
+    }
     // blocked layout: thread t owns items [t*kScanItems, (t+1)*kScanItems)
     const long first = base + static_cast<long>(threadIdx.x) * kScanItems;
     const bool whole = vec && first + kScanItems <= n;
@@ -136,6 +165,21 @@ scan_downsweep(const int *__restrict__ in, long n, const int *__restrict__ block
         for (int i = 0; i < kScanItems; ++i)
             if (first + i < n) out[first + i] = v[i];
     }
+}
+
+// The scan of n ints in launches on s; returns their number. Every CTA adding up the block sums
+// before it saves a launch while they are few; the additions grow with the square of n, so past
+// kManyBlocks (17M ints) one CTA scans the block sums first (400M row counts: 2.35 ms less of a
+// format conversion's 43.2; 24M and 40M the same either way).
+constexpr long kManyBlocks = 8192;
+int launch_scan(const int *in, int *out, long n, int *block_sums, bool vec, cudaStream_t s) {
+    const long nb = ceil_div(n, kScanChunk);
+    const unsigned grid = static_cast<unsigned>(nb);
+    const bool many = nb > kManyBlocks;
+    scan_reduce<<<grid, kThreads, 0, s>>>(in, n, block_sums);
+    if (many) scan_block_sums<<<1, kThreads, 0, s>>>(block_sums, nb);
+    scan_downsweep<<<grid, kThreads, 0, s>>>(in, n, block_sums, out, vec, many);
+    return many ? 3 : 2;
 }
 
 // One CTA, n <= kScanChunk: the scan in place in one launch.
@@ -475,12 +519,9 @@ size_t align256(size_t b) { return (b + 255) & ~size_t(255); }
 // Exclusive scan of n ints (in may equal out); `work` holds ceil(n / 2048) ints.
 static as_status exclusive_scan(as_ctx *ctx, const int *in, int *out, long n, int *work,
                                 cudaStream_t s) {
-    const long nb = ceil_div(n, kScanChunk);
-    if (nb == 0) return AS_OK;
-    scan_reduce<<<static_cast<unsigned>(nb), kThreads, 0, s>>>(in, n, work);
+    if (n == 0) return AS_OK;
     const bool vec = (reinterpret_cast<uintptr_t>(in) | reinterpret_cast<uintptr_t>(out)) % 16 == 0;
-    scan_downsweep<<<static_cast<unsigned>(nb), kThreads, 0, s>>>(in, n, work, out, vec);
-    ctx->launches += 2;
+    ctx->launches += launch_scan(in, out, n, work, vec, s);
     return check_cuda(cudaGetLastError(), "scan launch");
 }
 
@@ -538,9 +579,7 @@ static int sort_by_column(int M, int N, int nnz, const int *rowptr, const int *c
             scan_one_block<<<1, kThreads, 0, s>>>(w.hist, hist_n);
             launches += 1;
         } else {
-            scan_reduce<<<nb, kThreads, 0, s>>>(w.hist, hist_n, w.sums);
-            scan_downsweep<<<nb, kThreads, 0, s>>>(w.hist, hist_n, w.sums, w.hist, true);
-            launches += 2;
+            launches += launch_scan(w.hist, w.hist, hist_n, w.sums, true, s);
         }
         if (large)
             radix_scatter<kLargeItems><<<tiles, kSortThreads, smem, s>>>(
