@@ -529,15 +529,17 @@ as_status spmm_launch(as_ctx *ctx, int dtype, int variant, const SpmmArgs &a, cu
 }
 
 // Library choice for the fused pass, by entries and width, from sweeps on GB300 (graphs of 60k,
-// 574k, 15M and 35.8M entries, widths 8 to 256): the chunk is as long as leaves enough chunks to
-// fill the chip (a chunk is walked in order: 1024 entries take 0.2-0.3 ms by themselves, 128
-// about 50 us and 32 about 30 us; at 60k entries and width 48 in bf16 344 us with 1024, 30 with
-// 32; at 574k 315 with 1024, 62 with 128), and on a large graph narrow rows of B take the kernels
-// that bring several entries per load (35.8M entries, width 48, bf16: 2.55 ms with one entry per
-// warp step, 1.66 with two). Each class lists the narrowest tile first; a layout that none of a class
-// serves takes the 1024-entry kernels with 4- and 16-byte vectors, and one that those do not serve
-// is refused. Shorter chunks leave more carry slots: where the arena cannot hold them (the call is
-// being captured, or memory is short), the 1024-entry kernel runs.
+// 574k, 15M and 35.8M entries, widths 8 to 256). A chunk is walked in order (1024 entries take 0.2-0.3
+// ms by themselves, 128 about 50 us and 32 about 30 us), so it is short where the whole pass is:
+// at 60k entries and width 48 in bf16 344 us with 1024, 30 with 32; at 574k 315 with 1024, 62 with
+// 128. On a large graph narrow rows of B take the kernels that bring several entries per load
+// (35.8M entries, width 48, bf16: 2.55 ms with one entry per warp step, 1.66 with two). On either
+// side of the lines (0.2M, 0.29M and 0.32M entries, 1M, 3M, 4.95M and 5.1M, 10M; both types, 9
+// widths, uniform and power-law rows) no class was behind the 1024-entry kernels that served all sizes
+// before. Each class lists the narrowest tile first; a layout that none of a class serves takes the
+// 1024-entry kernels with 4- and 16-byte vectors, and one that those do not serve is refused.
+// Shorter chunks leave more carry slots: where the arena cannot hold them (the call is being
+// captured, or memory is short), the 1024-entry kernel runs, which sums rows in other places.
 struct FusedPick {
     int kind, vb, group, cpl, chunk, steps;
 };

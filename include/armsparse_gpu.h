@@ -201,10 +201,24 @@ as_status as_softmax_xent_bwd_bf16(as_ctx *ctx, int n, int C, const uint16_t *S,
  * CSC of A_fwd (colptr, rowind, values in CSC order), B = dOut, F = X and perm from
  * as_csr2csc_perm, it gives dX = A_fwd^T * dOut and the values' gradient in CSR order, gathering
  * dOut's rows once for both (separately, the SDDMM gathers a second time).
- * C follows the nnz-split SpMM variants (see as_spmm_csr_f32); each dA value is one FMA chain
- * per lane over the lane's columns, then a butterfly sum over the variant's lane group.
- * variant: 0 = library choice, else an nnz-split variant whose column tile (vector elements x
- * group x vectors per lane) covers N; others return AS_ERR_UNSUPPORTED. */
+ * C follows the entry-balanced SpMM variant that runs (see as_spmm_csr_f32): with an nnz-split
+ * variant a row inside one chunk is its CSR chain, a row over several the chunks' partial sums in a
+ * fixed order; a multi-entry variant ("nnzme") splits every row's sum over its sub-groups. Each dA
+ * value is one FMA chain per lane over the lane's columns, then a butterfly sum over the variant's
+ * lane group.
+ * variant: 0 = library choice, else an nnz-split or multi-entry variant whose column tile (vector
+ * elements x group x vectors per lane) covers N; others return AS_ERR_UNSUPPORTED.
+ * The library choice is by entries, width, type and alignment: below 300,000 entries chunks of 32
+ * (N up to 64) or 128 entries, below 5,000,000 chunks of 128, from there multi-entry kernels with
+ * chunks of 1024 (N up to 32 in FP32, 64 in bf16) or chunks of 256; layouts that these do not serve
+ * take chunks of 1024. So rows are summed in other places on either side of these sizes, and for
+ * large graphs with narrow rows no row is the CSR chain. Give a variant where the order has to be one
+ * and the same.
+ * Scratch: 2 * N floats and an int per chunk (35.8M entries at N = 256: 287 MB; 4.9M: 79 MB), held
+ * by the context, which grows and never shrinks, until it is destroyed. Where it cannot grow (the
+ * call is being captured and no call before it needed as much, or device memory is short) the
+ * library choice takes chunks of 1024, a quarter to a 32nd of the scratch, and with them their
+ * order: run the call once before capturing it to have the same bits. */
 as_status as_spmm_sddmm_csr_f32(as_ctx *ctx, int M, int K, int N, int nnz, const int *rowptr,
                                 const int *colind, const float *val, const float *B, long ldb,
                                 float *C, long ldc, float beta, const float *F, long ldf,
