@@ -58,9 +58,10 @@ vcsr4_count(int M, int nnz, const int *__restrict__ rowptr, const int *__restric
     int lo, hi;
     row_range(rowptr, static_cast<int>(w), nnz, status, lo, hi);
     int c = 0;
-    for (int e = lo + lane; e < hi; e += 32) {
+    // entries are counted unsigned here and below: one past the last of 2^31 - 1 is past the end
+    for (unsigned e = lo + lane; e < static_cast<unsigned>(hi); e += 32) {
         const int g = __ldg(colind + e) >> 2;
-        c += (e == lo) || (__ldg(colind + e - 1) >> 2) != g;  // a new group starts here
+        c += (e == static_cast<unsigned>(lo)) || (__ldg(colind + e - 1) >> 2) != g;  // a new group starts here
     }
 #pragma unroll
     for (int o = 16; o > 0; o >>= 1) c += __shfl_xor_sync(0xffffffffu, c, o);
@@ -78,12 +79,12 @@ vcsr4_fill(int M, int nnz, const int *__restrict__ rowptr, const int *__restrict
     row_range(rowptr, static_cast<int>(w), nnz, status, lo, hi);
     const int base = vrowptr[w];
     int started = 0;  // groups started in earlier batches of this row
-    for (int e0 = lo; e0 < hi; e0 += 32) {
-        const int e = e0 + lane;
-        const bool valid = e < hi;
+    for (unsigned e0 = lo; e0 < static_cast<unsigned>(hi); e0 += 32) {
+        const unsigned e = e0 + lane;
+        const bool valid = e < static_cast<unsigned>(hi);
         const int col = valid ? __ldg(colind + e) : 0;
         const int g = col >> 2;
-        const bool start = valid && ((e == lo) || (__ldg(colind + e - 1) >> 2) != g);
+        const bool start = valid && ((e == static_cast<unsigned>(lo)) || (__ldg(colind + e - 1) >> 2) != g);
         const unsigned m = __ballot_sync(0xffffffffu, start);
         const int bidx = started + __popc(m & ((2u << lane) - 1u)) - 1;  // this entry's block
         if (start) {
@@ -112,7 +113,7 @@ vcsr4_fill(int M, int nnz, const int *__restrict__ rowptr, const int *__restrict
 __device__ __forceinline__ int bsearch_col(const int *__restrict__ colind, int lo, int hi, int c) {
     // an index in [lo, hi) holding c, or -1
     while (lo < hi) {
-        const int mid = (lo + hi) >> 1;
+        const int mid = lo + ((hi - lo) >> 1);
         const int v = __ldg(colind + mid);
         if (v == c) return mid;
         if (v < c)
@@ -159,7 +160,7 @@ rowpair_count(int M, int nnz, const int *__restrict__ rowptr, const int *__restr
     int b0, b1;
     row_range(rowptr, static_cast<int>(ra + 1), nnz, status, b0, b1);
     int m = 0;
-    for (int f = b0 + lane; f < b1; f += 32) m += moved_b(colind, a0, a1, b0, b1, f);
+    for (unsigned f = b0 + lane; f < static_cast<unsigned>(b1); f += 32) m += moved_b(colind, a0, a1, b0, b1, f);
 #pragma unroll
     for (int o = 16; o > 0; o >>= 1) m += __shfl_xor_sync(0xffffffffu, m, o);
     if (lane == 0) {
@@ -184,9 +185,9 @@ rowpair_fill(int M, int nnz, const int *__restrict__ rowptr, const int *__restri
     // row a's segment: each entry, then its partner
     int pos = __ldg(rowptr2 + ra);
     const int end_a = __ldg(rowptr2 + ra + 1);
-    for (int i0 = a0; i0 < a1; i0 += 32) {
-        const int i = i0 + lane;
-        const bool valid = i < a1;
+    for (unsigned i0 = a0; i0 < static_cast<unsigned>(a1); i0 += 32) {
+        const unsigned i = i0 + lane;
+        const bool valid = i < static_cast<unsigned>(a1);
         const int f = valid && paired ? pair_of_a(colind, a0, a1, b0, b1, i) : -1;
         const unsigned mv = __ballot_sync(0xffffffffu, valid);
         const unsigned mp = __ballot_sync(0xffffffffu, f >= 0);
@@ -210,9 +211,9 @@ rowpair_fill(int M, int nnz, const int *__restrict__ rowptr, const int *__restri
     // row b's segment: its unmatched entries
     pos = __ldg(rowptr2 + ra + 1);
     const int end_b = __ldg(rowptr2 + ra + 2);
-    for (int f0 = b0; f0 < b1; f0 += 32) {
-        const int f = f0 + lane;
-        const bool keep = f < b1 && !moved_b(colind, a0, a1, b0, b1, f);
+    for (unsigned f0 = b0; f0 < static_cast<unsigned>(b1); f0 += 32) {
+        const unsigned f = f0 + lane;
+        const bool keep = f < static_cast<unsigned>(b1) && !moved_b(colind, a0, a1, b0, b1, f);
         const unsigned mk = __ballot_sync(0xffffffffu, keep);
         if (keep) {
             const int p = pos + __popc(mk & ((1u << lane) - 1u));

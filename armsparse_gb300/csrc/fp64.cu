@@ -40,7 +40,7 @@ sddmm_f64_kernel(int M, int N, int K, int nnz, const int *__restrict__ rowptr,
     if (e >= nnz) return;
     int lo = 0, hi = M;
     while (hi - lo > 1) {
-        const int mid = (lo + hi) >> 1;
+        const int mid = lo + ((hi - lo) >> 1);
         if (__ldg(rowptr + mid) <= e) lo = mid; else hi = mid;
     }
     const int r = lo, c = __ldg(colind + e);

@@ -182,7 +182,7 @@ sddmm_tc_kernel(const __grid_constant__ CUtensorMap tmXhi, const __grid_constant
             row_range(rowptr, row, nnz, status, lo, hi);
             int a = lo, b = hi;  // lower_bound of c0 in colind[lo, hi)
             while (a < b) {
-                const int m = (a + b) >> 1;
+                const int m = a + ((b - a) >> 1);
                 if (__ldg(colind + m) < c0)
                     a = m + 1;
                 else
@@ -483,7 +483,7 @@ sddmm_tc_persistent(const __grid_constant__ CUtensorMap tmXhi, const __grid_cons
                 row_range(rowptr, row, nnz, status, lo, hi);
                 int a = lo, b = hi;
                 while (a < b) {
-                    const int m = (a + b) >> 1;
+                    const int m = a + ((b - a) >> 1);
                     if (__ldg(colind + m) < c0) a = m + 1; else b = m;
                 }
                 e = a;
@@ -558,20 +558,21 @@ check_and_mark(int M, int N, int nnz, const int *__restrict__ rowptr,
         int lo, hi;
         row_range(rowptr, static_cast<int>(w), nnz, status, lo, hi);
         int carry = -1;  // column of the entry before this batch (-1 before the row's first)
-        for (int base = lo; base < hi; base += 128) {
+        const unsigned end = hi;  // unsigned: an entry past the last of 2^31 - 1 is past the end, not below zero
+        for (unsigned base = lo; base < end; base += 128) {
             int c[4];
 #pragma unroll
             for (int q = 0; q < 4; ++q) {
-                const int e = base + 32 * q + lane;
-                c[q] = e < hi ? __ldg(colind + e) : 0;
+                const unsigned e = base + 32 * q + lane;
+                c[q] = e < end ? __ldg(colind + e) : 0;
             }
 #pragma unroll
             for (int q = 0; q < 4; ++q) {
-                const int e = base + 32 * q + lane;
+                const unsigned e = base + 32 * q + lane;
                 const int up = __shfl_up_sync(0xffffffffu, c[q], 1);
                 const int last = __shfl_sync(0xffffffffu, c[q], 31);
                 const int prev = lane == 0 ? carry : up;
-                if (e < hi) {
+                if (e < end) {
                     if (c[q] < 0 || c[q] >= N || prev >= c[q])
                         bad = true;
                     else if (prev < 0 || prev / BN != c[q] / BN)
@@ -683,9 +684,9 @@ check_sorted_rows(int M, int N, int nnz, const int *__restrict__ rowptr,
     int lo, hi;
     row_range(rowptr, static_cast<int>(w), nnz, status, lo, hi);
     bool bad = false;
-    for (int e = lo + lane; e < hi; e += 32) {
+    for (unsigned e = lo + lane; e < static_cast<unsigned>(hi); e += 32) {
         const int c = __ldg(colind + e);
-        if (c < 0 || c >= N || (e > lo && __ldg(colind + e - 1) >= c)) bad = true;
+        if (c < 0 || c >= N || (e > static_cast<unsigned>(lo) && __ldg(colind + e - 1) >= c)) bad = true;
     }
     if (__any_sync(0xffffffffu, bad) && lane == 0) flag(status, kFlagBadColind);
 }

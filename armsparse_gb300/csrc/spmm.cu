@@ -117,10 +117,12 @@ spmm_rowsplit(int M, int K, int N, int nnz, const int *__restrict__ rowptr,
 
     // (colind, val) of GROUP entries per batch, one per lane. PF: the next batch is loaded while
     // the current one is consumed (registers capped so that four CTAs stay resident)
-    auto load_entry = [&](int e, int &k, float &v) {
+    // (unsigned: an entry ahead of 2^31 - 1 of them is past the end, not below zero)
+    const unsigned end = hi;
+    auto load_entry = [&](unsigned e, int &k, float &v) {
         k = -1;
         v = 0.0f;
-        if (e < hi) {
+        if (e < end) {
             k = ld_stream(colind + e);
             v = to_f32(ld_stream(val + e));
             if (static_cast<unsigned>(k) >= static_cast<unsigned>(K)) {
@@ -131,8 +133,8 @@ spmm_rowsplit(int M, int K, int N, int nnz, const int *__restrict__ rowptr,
     };
     int kn = -1;
     float vn = 0.0f;
-    if (PF) load_entry(lo + g, kn, vn);
-    for (int base = lo; base < hi; base += GROUP) {
+    if (PF) load_entry(static_cast<unsigned>(lo) + g, kn, vn);
+    for (unsigned base = lo; base < end; base += GROUP) {
         int k;
         float v;
         if (PF) {
@@ -142,7 +144,7 @@ spmm_rowsplit(int M, int K, int N, int nnz, const int *__restrict__ rowptr,
         } else {
             load_entry(base + g, k, v);
         }
-        const int cnt = min(GROUP, hi - base);
+        const int cnt = static_cast<int>(min(static_cast<unsigned>(GROUP), end - base));
         // U entries per step: their B loads are issued before the FMAs, which then run in
         // CSR order. fp32 keeps per-load predicates (measured faster on GB300); bf16 loads
         // branch-free into packed registers (an idle lane or a flagged entry reads an

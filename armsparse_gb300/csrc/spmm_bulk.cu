@@ -136,10 +136,10 @@ spmm_bulk(int M, int K, int N, int nnz, const int *__restrict__ rowptr,
     const int n = hi - lo;
     // batches of 32 (colind, val): current and next, lane i holds entry 32*b + i
     auto load_batch = [&](int b, int &k, float &v) {
-        const int e = lo + 32 * b + lane;
+        const unsigned e = lo + 32u * b + lane;  // unsigned: an entry past the last of 2^31 - 1 is past the end, not below zero
         k = -1;
         v = 0.0f;
-        if (e < hi) {
+        if (e < static_cast<unsigned>(hi)) {
             k = ld_stream(colind + e);
             v = to_f32(ld_stream(val + e));
             if (static_cast<unsigned>(k) >= static_cast<unsigned>(K)) {

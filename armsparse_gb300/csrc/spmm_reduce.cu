@@ -49,11 +49,12 @@ spmm_reduce(int M, int K, int N, int nnz, const int *__restrict__ rowptr,
     for (int j = 0; j < CPL; ++j)
 #pragma unroll
         for (int i = 0; i < E; ++i) acc[j][i] = OP == 0 ? 0.0f : OP == 1 ? -INFINITY : -10000.0f;
-    for (int base = lo; base < hi; base += 32) {
-        const int e = base + lane;
+    const unsigned end = hi;  // unsigned: an entry past the last of 2^31 - 1 is past the end, not below zero
+    for (unsigned base = lo; base < end; base += 32) {
+        const unsigned e = base + lane;
         int k = -1;
         float w = 1.0f;
-        if (e < hi) {
+        if (e < end) {
             k = ld_stream(colind + e);
             if (WEIGHTED) w = ld_stream(val + e);
             if (static_cast<unsigned>(k) >= static_cast<unsigned>(K)) {
@@ -61,7 +62,7 @@ spmm_reduce(int M, int K, int N, int nnz, const int *__restrict__ rowptr,
                 k = -1;
             }
         }
-        const int cnt = min(32, hi - base);
+        const int cnt = static_cast<int>(min(32u, end - base));
         for (int t = 0; t < cnt; ++t) {
             const int kk = __shfl_sync(0xffffffffu, k, t);
             const float ww = __shfl_sync(0xffffffffu, w, t);

@@ -92,11 +92,12 @@ spmm_rowpair(int M, int K, int N, int nnz, const int *__restrict__ rowptr2,
         for (int j = 0; j < CPL; ++j)
 #pragma unroll
             for (int i = 0; i < E; ++i) b[j][i] = 0.0f;  // what a flagged first entry reuses
-        for (int base = lo; base < hi; base += 32) {
-            const int e = base + lane;
+        const unsigned end = hi;  // unsigned: an entry past the last of 2^31 - 1 is past the end, not below zero
+        for (unsigned base = lo; base < end; base += 32) {
+            const unsigned e = base + lane;
             int k = -1, f = 0;
             float v = 0.0f;
-            if (e < hi) {
+            if (e < end) {
                 k = ld_stream(colind2 + e);
                 v = ld_stream(val2 + e);
                 f = honour && __ldg(flag2 + e) != 0;
@@ -105,7 +106,7 @@ spmm_rowpair(int M, int K, int N, int nnz, const int *__restrict__ rowptr2,
                     k = -1;
                 }
             }
-            const int cnt = min(32, hi - base);
+            const int cnt = static_cast<int>(min(32u, end - base));
             for (int t = 0; t < cnt; ++t) {
                 const int kk = __shfl_sync(0xffffffffu, k, t);
                 const float vv = __shfl_sync(0xffffffffu, v, t);

@@ -51,11 +51,12 @@ spmm_vcsr4(int M, int K, int N, int nslots, const int *__restrict__ vrowptr,
         for (int i = 0; i < E; ++i)
             acc[j][i] = (beta != 0.0f && c < N) ? C[row * ldc + c + i] * beta : 0.0f;
     }
-    for (int base = lo; base < hi; base += 32) {
-        const int e = base + lane;
+    const unsigned end = hi;  // unsigned: an entry past the last of 2^31 - 1 is past the end, not below zero
+    for (unsigned base = lo; base < end; base += 32) {
+        const unsigned e = base + lane;
         int k = -1;
         float v = 0.0f;
-        if (e < hi) {
+        if (e < end) {
             k = ld_stream(vcolind + e);
             v = ld_stream(vval + e);
             if (static_cast<unsigned>(k) >= static_cast<unsigned>(K)) {
@@ -63,7 +64,7 @@ spmm_vcsr4(int M, int K, int N, int nslots, const int *__restrict__ vrowptr,
                 k = -1;
             }
         }
-        const int cnt = min(32, hi - base);
+        const int cnt = static_cast<int>(min(32u, end - base));
         for (int t = 0; t < cnt; ++t) {
             const int kk = __shfl_sync(0xffffffffu, k, t);
             const float vv = __shfl_sync(0xffffffffu, v, t);

@@ -48,8 +48,9 @@ spmv_csr(int M, int K, int nnz, const int *__restrict__ rowptr, const int *__res
     }
     // lane g sums its entries g, g + GROUP, ... in order, four gathers in flight
     float s = 0.0f;
-    int e = lo + g;
-    for (; e + 3 * GROUP < hi; e += 4 * GROUP) {
+    const unsigned end = hi;  // unsigned: an entry past the last of 2^31 - 1 is past the end, not below zero
+    unsigned e = static_cast<unsigned>(lo) + g;
+    for (; e + 3 * GROUP < end; e += 4 * GROUP) {
         int k[4];
         float v[4], xv[4];
 #pragma unroll
@@ -68,7 +69,7 @@ spmv_csr(int M, int K, int nnz, const int *__restrict__ rowptr, const int *__res
         for (int u = 0; u < 4; ++u)
             if (k[u] >= 0) s = fmaf(v[u], xv[u], s);
     }
-    for (; e < hi; e += GROUP) {
+    for (; e < end; e += GROUP) {
         const int k = ld_stream(colind + e);
         if (static_cast<unsigned>(k) >= static_cast<unsigned>(K)) {
             flag(status, kFlagBadColind);
@@ -106,8 +107,9 @@ spmv_vcsr4(int M, int K, int nslots, const int *__restrict__ rowptr,
         return;
     }
     float s = 0.f;
-    int idx = lo;
-    for (; idx + 4 * U <= hi; idx += 4 * U) {
+    const unsigned end = hi;  // unsigned, as above
+    unsigned idx = lo;
+    for (; idx + 4 * U <= end; idx += 4 * U) {
         int k[U];
         float v[U], xv[U];
 #pragma unroll
@@ -128,7 +130,7 @@ spmv_vcsr4(int M, int K, int nslots, const int *__restrict__ rowptr,
         for (int u = 0; u < U; ++u)
             if (k[u] >= 0) s = fmaf(v[u], xv[u], s);
     }
-    for (; idx < hi; idx += 4) {
+    for (; idx < end; idx += 4) {
         const int k = ld_stream(colind + idx);
         if (k < 0 || k > K - 4) {
             flag(status, kFlagBadColind);
@@ -169,8 +171,9 @@ spmv_long(int M, int K, int nnz, const int *__restrict__ rowptr, const int *__re
         if (MODE == 0) {
             // thread t sums entries lo + t, lo + t + 256, ... in order, four gathers in flight
             float s = 0.0f;
-            int e = lo + tid;
-            for (; e + 3 * kThreads < hi; e += 4 * kThreads) {
+            const unsigned end = hi;
+            unsigned e = static_cast<unsigned>(lo) + tid;
+            for (; e + 3 * kThreads < end; e += 4 * kThreads) {
                 int k[4];
                 float v[4], xv[4];
 #pragma unroll
@@ -189,7 +192,7 @@ spmv_long(int M, int K, int nnz, const int *__restrict__ rowptr, const int *__re
                 for (int u = 0; u < 4; ++u)
                     if (k[u] >= 0) s = fmaf(v[u], xv[u], s);
             }
-            for (; e < hi; e += kThreads) {
+            for (; e < end; e += kThreads) {
                 const int k = ld_stream(colind + e);
                 if (static_cast<unsigned>(k) >= static_cast<unsigned>(K)) {
                     flag(status, kFlagBadColind);
@@ -216,8 +219,8 @@ spmv_long(int M, int K, int nnz, const int *__restrict__ rowptr, const int *__re
             // threads [t0, kThreads)
             auto stage = [&](int j, int t0) {
                 for (int i = tid - t0; i < kThreads; i += kThreads - t0) {
-                    const int b = lo + 4 * (j * kThreads + i);
-                    if (b >= hi) break;
+                    const unsigned b = lo + 4u * (j * kThreads + i);
+                    if (b >= static_cast<unsigned>(hi)) break;
                     const int k = ld_stream(colind + b);
                     const bool ok = k >= 0 && k <= K - 4;
                     if (!ok) flag(status, kFlagBadColind);

@@ -64,3 +64,40 @@ def test_spgemm_reads_no_entry_past_the_last(length):
     A.sync_status()
     rest = [0.0] * (80 - length)
     assert C.tolist() == [[2.0] * length + rest, [3.0] * length + rest]
+
+
+def test_row_kernels_read_no_entry_past_the_last():
+    """Rows of at most 256 entries, the last of 250 (no whole number of steps)."""
+    lens = torch.full((2 ** 23 + 1,), 256, dtype=torch.int64, device=dev())
+    lens[0], lens[1], lens[-1] = 6, 255, 250
+    rp = torch.zeros(lens.numel() + 1, dtype=torch.int32, device=dev())
+    rp[1:] = torch.cumsum(lens, 0)
+    assert int(rp[-1]) == NNZ
+    ci, v = _columns(), torch.ones(NNZ, device=dev())
+    B = torch.zeros(2, 8, device=dev())
+    B[1] = torch.arange(8)
+
+    def check(C, last):
+        A.sync_status()
+        assert C[-1].tolist() == last and not C[:-1].any()
+
+    total = [3.0 * i for i in range(8)]
+    check(A.spmm(rp, ci, v, B), total)
+    check(A.spmm(rp, ci, v, B, variant=A.spmm_variants().index("rowsplit_v8_g32_c4_u4_pf") + 1), total)
+    check(A.spmm_reduce(rp, ci, B, op="sum"), total)
+    check(A.spmm_reduce(rp, ci, B, val=v, op="max"), [float(i) for i in range(8)])
+    check(A.spmv(rp, ci, v, torch.tensor([0.0, 2.0], device=dev()))[:, None], [6.0])
+    flags = torch.zeros(NNZ, dtype=torch.uint8, device=dev())
+    check(A.spmm_rowpair(rp, ci, v, flags, B), total)
+
+
+def test_row_pairs_of_a_matrix_past_half_the_limit():
+    """The search for a column in a row's second half, past 2^30 entries."""
+    rows = 2 ** 20 + 2 ** 18
+    rp = torch.arange(rows + 1, dtype=torch.int32, device=dev()) * 1024
+    ci = (torch.arange(1024, dtype=torch.int32, device=dev())).repeat(rows)
+    rp2, ci2, _, flag2 = A.csr_to_rowpair(rp, ci, torch.ones(rows * 1024, device=dev()))
+    A.sync_status()
+    # both rows of a pair hold the same columns: the first takes all of its partner's entries
+    assert torch.equal(rp2[::2], rp[::2]) and torch.equal(rp2[1:-1:2], rp[2::2])
+    assert ci2[-4:].tolist() == [1022, 1022, 1023, 1023] and flag2[-4:].tolist() == [0, 1, 0, 1]
