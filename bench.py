@@ -90,7 +90,7 @@ class SpmmF32(Workload):
     metric = "SpMM GB/s (algorithmic bytes) and % HBM roofline"
     unit = "GB/s"
     dtype = "f32"
-    kernel = "spmm_rowsplit (the call; its long-row kernel finds no long row here)"
+    kernel = "spmm_rowsplit (the call; its long-row kernel finds no row over 256 entries here)"
     profile = "spmm_rowsplit_f32_4096x4096x4096_d001"
     e2e_api = "libarmsparse_drivers.so origin() (SDMM.cpp:422 signature) with host buffers"
 
