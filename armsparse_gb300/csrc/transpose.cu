@@ -44,7 +44,10 @@ constexpr int kSortThreads = 512;   // of a tile's CTA
 constexpr int kSortWarps = kSortThreads / 32;
 constexpr int kLargeItems = 8;      // entries per thread of a tile
 constexpr int kSmallItems = 2;
-constexpr int kLargeNnz = 300000;   // from here on large tiles (1M entries: 81 us, small ones 96)
+// From here on large tiles. Both, on square, narrow and wide matrices: 100,000 entries 41-72 us with
+// small tiles, 39-80 with large ones; 300,000 43-67 and 47-74; 350,000 to 400,000 the same within 4 %;
+// 500,000 49-79 and 47-74; 1M 62-97 and 53-84.
+constexpr int kLargeNnz = 300000;
 constexpr int kBins = 256;          // digits per pass at most
 
 // ---- exclusive scan of int32 (three phases, no cross-CTA waits) ---------------------------
